@@ -13,7 +13,7 @@ set -euo pipefail
 REF=${1:-${LNT_REFERENCE_DIR:-/root/reference}}
 HERE=$(cd "$(dirname "$0")" && pwd)
 OUT="$HERE/_ref"
-if [ ! -d "$REF" ]; then
+if [ ! -d "$REF" ] || [ -z "$(find "$REF" -type f \( -name '*.cu' -o -name '*.cpp' \) -print -quit)" ]; then
     echo "build_ref: no reference sources at $REF; keeping the prebuilt binary if any"
     exit 0
 fi
