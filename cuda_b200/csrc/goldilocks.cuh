@@ -270,6 +270,15 @@ GL_HD uint64_t mul(uint64_t a, uint64_t b) {
 #endif
 }
 
+// any 64-bit word to [0, p)
+GL_HD uint64_t canon(uint64_t a) {
+#if defined(__CUDA_ARCH__)
+  return canon_words((uint32_t)a, (uint32_t)(a >> 32));
+#else
+  return a >= P ? a - P : a;
+#endif
+}
+
 GL_HD uint64_t sqr(uint64_t a) { return mul(a, a); }
 
 GL_HD uint64_t pow(uint64_t a, uint64_t e) {

@@ -1,0 +1,377 @@
+// Lazily reduced transforms of up to 16 points with power-of-two roots: the
+// register butterflies of the pass kernels (smem_passes.cuh).
+//
+// Between the general multiplications of a pass nothing needs a residue in
+// [0, p).  Here a value inside a butterfly network is a signed 96-bit integer in
+// three 32-bit words (W3), congruent to the residue: an addition is one carry
+// chain of three instructions and no correction, a multiplication by 2^24, 2^48
+// or 2^72 a few shifts with 2^96 = -1 and 2^64 = 2^32 - 1 folded in.  A word is
+// brought back below 2^64 once per pass (reduce), congruent but not canonical:
+// every consumer is a product or another network, which take any 64-bit word.
+//
+// Cost of an 8-point transform: 72 instructions of additions, 42 of shifts, 51 of bias and
+// reduction, against 273 with canonical additions (ntt_core.cuh).  The kernels are bound by
+// integer issue (ALU and multiplier pipes 50-65 % busy, HBM 14 %): at n = 2^23 a squaring took
+// 441.2 us with canonical values and takes 363.1 us with these (row_square 210.5 -> 161.5,
+// col_fused 240.8 -> 212.2); n = 2048 on one SM 10.15 -> 8.99 us.
+//
+// Ranges.  Inputs of a network: |x| < 2^66 (a 64-bit word, or the three words of
+// mul3, in (-2^32, 2^65)).  Differences are then below 2^67, times 2^24 below
+// 2^91, and no sum passes 2^93: three words never overflow.  The bias kBias p
+// (2^28 p, congruent to 0) is added to input 0, which reaches every output with
+// coefficient +1, so every output is non-negative and below 2^93.
+//
+// On the host the same formulas run on 128-bit integers and check those ranges
+// (tests/native/lazy_selftest.cpp).
+#pragma once
+#include <stdint.h>
+
+#include "goldilocks.cuh"
+#include "ntt_core.cuh"
+
+namespace lnt {
+namespace lazy {
+
+// a0 + a1 2^32 + a2 2^64 with a2 signed
+struct W3 {
+  uint32_t a0, a1, a2;
+};
+
+constexpr uint32_t kBias = 1u << 28;
+
+GL_HD W3 from_word(uint64_t x) { return {(uint32_t)x, (uint32_t)(x >> 32), 0u}; }
+
+#if !defined(__CUDA_ARCH__)
+inline __int128 to_int(const W3& x) {
+  return ((__int128)(int32_t)x.a2 << 64) + (__int128)(((uint64_t)x.a1 << 32) | x.a0);
+}
+// a value outside 96 bits is an error of the ranges above; the selftest reads this
+inline bool& range_error() {
+  static bool bad = false;
+  return bad;
+}
+inline W3 from_int(__int128 v) {
+  const __int128 lim = (__int128)1 << 95;
+  if (v >= lim || v < -lim) range_error() = true;
+  return {(uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64)};
+}
+#endif
+
+GL_HD W3 add(const W3& x, const W3& y) {
+#if defined(__CUDA_ARCH__)
+  W3 r;
+  asm("add.cc.u32 %0, %3, %6;\n\t"
+      "addc.cc.u32 %1, %4, %7;\n\t"
+      "addc.u32 %2, %5, %8;"
+      : "=r"(r.a0), "=r"(r.a1), "=r"(r.a2)
+      : "r"(x.a0), "r"(x.a1), "r"(x.a2), "r"(y.a0), "r"(y.a1), "r"(y.a2));
+  return r;
+#else
+  return from_int(to_int(x) + to_int(y));
+#endif
+}
+
+GL_HD W3 sub(const W3& x, const W3& y) {
+#if defined(__CUDA_ARCH__)
+  W3 r;
+  asm("sub.cc.u32 %0, %3, %6;\n\t"
+      "subc.cc.u32 %1, %4, %7;\n\t"
+      "subc.u32 %2, %5, %8;"
+      : "=r"(r.a0), "=r"(r.a1), "=r"(r.a2)
+      : "r"(x.a0), "r"(x.a1), "r"(x.a2), "r"(y.a0), "r"(y.a1), "r"(y.a2));
+  return r;
+#else
+  return from_int(to_int(x) - to_int(y));
+#endif
+}
+
+// x + kBias p
+GL_HD W3 add_bias(const W3& x) {
+  return add(x, W3{kBias, 0u - kBias, kBias - 1u});
+}
+
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ uint32_t sign_word(uint32_t a2) { return (uint32_t)((int32_t)a2 >> 31); }
+#endif
+
+// x 2^24, |x| < 2^67
+GL_HD W3 mul_2_24(const W3& x) {
+#if defined(__CUDA_ARCH__)
+  return {x.a0 << 24, __funnelshift_l(x.a0, x.a1, 24), __funnelshift_l(x.a1, x.a2, 24)};
+#else
+  return from_int(to_int(x) * ((__int128)1 << 24));
+#endif
+}
+
+// x 2^48, |x| < 2^79.  With (l2 : l1 : l0) = x 2^16 it is l0 2^32 + l1 2^64 + l2 2^96 =
+// l0 2^32 + l1 (2^32 - 1) - l2.
+GL_HD W3 mul_2_48(const W3& x) {
+#if defined(__CUDA_ARCH__)
+  const uint32_t l0 = x.a0 << 16, l1 = __funnelshift_l(x.a0, x.a1, 16), l2 = __funnelshift_l(x.a1, x.a2, 16);
+  const uint32_t sg = sign_word(x.a2);
+  W3 r;
+  asm("mad.lo.cc.u32  %0, %4, 0xFFFFFFFF, 0;\n\t"
+      "madc.hi.cc.u32 %1, %4, 0xFFFFFFFF, %3;\n\t"
+      "addc.u32       %2, 0, 0;\n\t"
+      "sub.cc.u32     %0, %0, %5;\n\t"
+      "subc.cc.u32    %1, %1, %6;\n\t"
+      "subc.u32       %2, %2, %6;"
+      : "=&r"(r.a0), "=&r"(r.a1), "=&r"(r.a2)
+      : "r"(l0), "r"(l1), "r"(l2), "r"(sg));
+  return r;
+#else
+  const __int128 l = to_int(x) * 65536;
+  const __int128 l0 = (uint32_t)l, l1 = (uint32_t)(l >> 32), l2 = l >> 64;
+  return from_int((l0 << 32) + l1 * 0xFFFFFFFFll - l2);
+#endif
+}
+
+// x 2^72, |x| < 2^87.  With (e2 : e1 : e0) = x 2^8 it is e0 2^64 + e1 2^96 + e2 2^128 =
+// (e0 - e2) 2^32 - e0 - e1.
+GL_HD W3 mul_2_72(const W3& x) {
+#if defined(__CUDA_ARCH__)
+  const uint32_t e0 = x.a0 << 8, e1 = __funnelshift_l(x.a0, x.a1, 8), e2 = __funnelshift_l(x.a1, x.a2, 8);
+  const uint32_t sg = sign_word(x.a2);
+  W3 r;
+  asm("sub.cc.u32  %0, 0, %3;\n\t"
+      "subc.cc.u32 %1, %3, %5;\n\t"
+      "subc.u32    %2, 0, %6;\n\t"
+      "sub.cc.u32  %0, %0, %4;\n\t"
+      "subc.cc.u32 %1, %1, 0;\n\t"
+      "subc.u32    %2, %2, 0;"
+      : "=&r"(r.a0), "=&r"(r.a1), "=&r"(r.a2)
+      : "r"(e0), "r"(e1), "r"(e2), "r"(sg));
+  return r;
+#else
+  const __int128 e = to_int(x) * 256;
+  const __int128 e0 = (uint32_t)e, e1 = (uint32_t)(e >> 32), e2 = e >> 64;
+  return from_int((e0 - e2) * ((__int128)1 << 32) - e0 - e1);
+#endif
+}
+
+// 0 <= x < 2^95 to a congruent 64-bit word: (a1 : a0) + a2 (2^32 - 1), whose carry c
+// comes back as c (2^32 - 1): with c = 1 the wrapped sum is below 2^63, so that cannot wrap.
+GL_HD uint64_t reduce(const W3& x) {
+#if defined(__CUDA_ARCH__)
+  uint32_t t0, t1;
+  asm("{\n\t"
+      ".reg .u32 c;\n\t"
+      "mad.lo.cc.u32  %0, %4, 0xFFFFFFFF, %2;\n\t"
+      "madc.hi.cc.u32 %1, %4, 0xFFFFFFFF, %3;\n\t"
+      "addc.u32       c, 0, 0;\n\t"
+      "add.u32        %1, %1, c;\n\t"
+      "sub.cc.u32     %0, %0, c;\n\t"
+      "subc.u32       %1, %1, 0;\n\t"
+      "}"
+      : "=&r"(t0), "=&r"(t1)
+      : "r"(x.a0), "r"(x.a1), "r"(x.a2));
+  return ((uint64_t)t1 << 32) | t0;
+#else
+  const __int128 v = to_int(x);
+  if (v < 0) range_error() = true;
+  const __int128 s = (v & (((__int128)1 << 64) - 1)) + (v >> 64) * 0xFFFFFFFFll;
+  const __int128 r = (s & (((__int128)1 << 64) - 1)) + (s >> 64) * 0xFFFFFFFFll;
+  if (r >> 64) range_error() = true;
+  return (uint64_t)r;
+#endif
+}
+
+// x in (-p, 2^65 - 2^33] (a2 = -1, 0 or 1) to a congruent 64-bit word:
+// (a1 : a0) + a2 (2^32 - 1), which can neither carry nor borrow again.
+GL_HD uint64_t fold(const W3& x) {
+#if defined(__CUDA_ARCH__)
+  const uint32_t sg = sign_word(x.a2);
+  uint32_t t0, t1;
+  asm("{\n\t"
+      "add.u32     %1, %3, %4;\n\t"
+      "sub.cc.u32  %0, %2, %4;\n\t"
+      "subc.u32    %1, %1, %5;\n\t"
+      "}"
+      : "=&r"(t0), "=&r"(t1)
+      : "r"(x.a0), "r"(x.a1), "r"(x.a2), "r"(sg));
+  return ((uint64_t)t1 << 32) | t0;
+#else
+  const __int128 v = to_int(x);
+  const __int128 r = (v & (((__int128)1 << 64) - 1)) + (v >> 64) * 0xFFFFFFFFll;
+  if (r < 0 || (r >> 64)) range_error() = true;
+  return (uint64_t)r;
+#endif
+}
+
+// a b for any 64-bit words, in (-2^32, 2^65 - 2^33]: with the product's 32-bit words r0..r3,
+// (r1 : r0) + r2 (2^32 - 1) - r3.  The outer products are plain wide ones and the cross
+// products one chain with a carry, added in on the integer ALU: 17 instructions with the fold of
+// mul, against 22 when every partial product is a multiply-add of the one before (the
+// multiplier pipe is the fuller one there); at n = 2^23 363.1 against 375.4 us a squaring.
+GL_HD W3 mul3(uint64_t a, uint64_t b) {
+#if defined(__CUDA_ARCH__)
+  W3 t;
+  asm("{\n\t"
+      ".reg .u32 r0, r1, r2, r3, u0, u1;\n\t"
+      ".reg .u64 q0, q3;\n\t"
+      "mul.wide.u32   q0, %3, %5;\n\t"
+      "mul.wide.u32   q3, %4, %6;\n\t"
+      "mul.lo.u32     u0, %3, %6;\n\t"
+      "mul.hi.u32     u1, %3, %6;\n\t"
+      "mov.b64        {r0, r1}, q0;\n\t"
+      "mov.b64        {r2, r3}, q3;\n\t"
+      "mad.lo.cc.u32  u0, %4, %5, u0;\n\t"
+      "madc.hi.cc.u32 u1, %4, %5, u1;\n\t"
+      "addc.u32       r3, r3, 0;\n\t"
+      "add.cc.u32     r1, r1, u0;\n\t"
+      "addc.cc.u32    r2, r2, u1;\n\t"
+      "addc.u32       r3, r3, 0;\n\t"
+      "mad.lo.cc.u32  %0, r2, 0xFFFFFFFF, r0;\n\t"
+      "madc.hi.cc.u32 %1, r2, 0xFFFFFFFF, r1;\n\t"
+      "addc.u32       %2, 0, 0;\n\t"
+      "sub.cc.u32     %0, %0, r3;\n\t"
+      "subc.cc.u32    %1, %1, 0;\n\t"
+      "subc.u32       %2, %2, 0;\n\t"
+      "}"
+      : "=&r"(t.a0), "=&r"(t.a1), "=&r"(t.a2)
+      : "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"((uint32_t)b), "r"((uint32_t)(b >> 32)));
+  return t;
+#else
+  const unsigned __int128 q = (unsigned __int128)a * b;
+  const __int128 lo = (uint64_t)q, r2 = (uint32_t)(uint64_t)(q >> 64), r3 = (uint64_t)(q >> 96);
+  return from_int(lo + r2 * 0xFFFFFFFFll - r3);
+#endif
+}
+
+// a b as a 64-bit word (congruent, not canonical)
+GL_HD uint64_t mul(uint64_t a, uint64_t b) { return fold(mul3(a, b)); }
+
+// ---- transforms: x (natural order, overwritten) -> out (bit-reversed order), and back ----
+
+// natural in, bit-reversed out, root 2^(192/R)
+template <int R>
+GL_HD void dif(W3 (&x)[R], uint64_t (&out)[R]) {
+  static_assert(R == 2 || R == 4 || R == 8 || R == 16, "register transform size");
+  if constexpr (R == 2) {
+    const W3 a = add_bias(x[0]);
+    out[0] = reduce(add(a, x[1]));
+    out[1] = reduce(sub(a, x[1]));
+  } else if constexpr (R == 4) {
+    const W3 a = add_bias(x[0]);
+    const W3 s0 = add(a, x[2]), d0 = sub(a, x[2]), s1 = add(x[1], x[3]);
+    const W3 d1 = mul_2_48(sub(x[1], x[3]));
+    out[0] = reduce(add(s0, s1));
+    out[1] = reduce(sub(s0, s1));
+    out[2] = reduce(add(d0, d1));
+    out[3] = reduce(sub(d0, d1));
+  } else if constexpr (R == 8) {
+    const W3 a = add_bias(x[0]);
+    const W3 s0 = add(a, x[4]), d0 = sub(a, x[4]);
+    const W3 s2 = add(x[2], x[6]), d2 = mul_2_48(sub(x[2], x[6]));
+    const W3 s1 = add(x[1], x[5]), d1 = sub(x[1], x[5]);
+    const W3 s3 = add(x[3], x[7]), d3 = sub(x[3], x[7]);
+    {
+      const W3 e0 = add(s0, s2), e1 = add(s1, s3);
+      out[0] = reduce(add(e0, e1));
+      out[1] = reduce(sub(e0, e1));
+      const W3 e2 = sub(s0, s2), e3 = mul_2_48(sub(s1, s3));
+      out[2] = reduce(add(e2, e3));
+      out[3] = reduce(sub(e2, e3));
+    }
+    // frequencies 1, 5: 2^24 (d1 + 2^48 d3); 3, 7: 2^72 (d1 - 2^48 d3) = 2^72 d1 + 2^24 d3
+    {
+      const W3 f = add(d0, d2), y = add(mul_2_24(d1), mul_2_72(d3));
+      out[4] = reduce(add(f, y));
+      out[5] = reduce(sub(f, y));
+    }
+    {
+      const W3 f = sub(d0, d2), y = add(mul_2_72(d1), mul_2_24(d3));
+      out[6] = reduce(add(f, y));
+      out[7] = reduce(sub(f, y));
+    }
+  } else {
+    // one stage with the twiddles 2^(12 k), its differences reduced to words, then two 8-point halves
+    W3 h[8];
+    uint64_t o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      h[k] = add(x[k], x[k + 8]);
+      x[k + 8] = sub(x[k], x[k + 8]);
+    }
+    dif<8>(h, o);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[k] = o[k];
+    h[0] = x[8];
+    h[1] = from_word(shl_c<12>(reduce(add_bias(x[9]))));
+    h[2] = from_word(shl_c<24>(reduce(add_bias(x[10]))));
+    h[3] = from_word(shl_c<36>(reduce(add_bias(x[11]))));
+    h[4] = from_word(shl_c<48>(reduce(add_bias(x[12]))));
+    h[5] = from_word(shl_c<60>(reduce(add_bias(x[13]))));
+    h[6] = from_word(shl_c<72>(reduce(add_bias(x[14]))));
+    h[7] = from_word(shl_c<84>(reduce(add_bias(x[15]))));
+    dif<8>(h, o);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[8 + k] = o[k];
+  }
+}
+
+// bit-reversed in, natural out, inverse root, unscaled
+template <int R>
+GL_HD void dit_inv(W3 (&x)[R], uint64_t (&out)[R]) {
+  static_assert(R == 2 || R == 4 || R == 8 || R == 16, "register transform size");
+  if constexpr (R == 2) {
+    dif<2>(x, out);
+  } else if constexpr (R == 4) {
+    const W3 a = add_bias(x[0]);
+    const W3 p0 = add(a, x[1]), p1 = sub(a, x[1]), p2 = add(x[2], x[3]);
+    const W3 p3 = mul_2_48(sub(x[2], x[3]));
+    out[0] = reduce(add(p0, p2));
+    out[2] = reduce(sub(p0, p2));
+    out[1] = reduce(sub(p1, p3));
+    out[3] = reduce(add(p1, p3));
+  } else if constexpr (R == 8) {
+    const W3 a = add_bias(x[0]);
+    const W3 p0 = add(a, x[1]), p1 = sub(a, x[1]);
+    const W3 p2 = add(x[2], x[3]), p3 = mul_2_48(sub(x[2], x[3]));
+    const W3 q0 = add(x[4], x[5]), q1 = sub(x[4], x[5]);
+    const W3 q2 = add(x[6], x[7]), q3 = sub(x[6], x[7]);
+    {
+      const W3 e = add(p0, p2), f = add(q0, q2);
+      out[0] = reduce(add(e, f));
+      out[4] = reduce(sub(e, f));
+      const W3 g = sub(p0, p2), h = mul_2_48(sub(q0, q2));  // inverse twiddle 2^-48 = -2^48
+      out[2] = reduce(sub(g, h));
+      out[6] = reduce(add(g, h));
+    }
+    {
+      // 2^-24 (q1 - 2^48 q3) = -2^72 (q1 - 2^48 q3) = -(2^72 q1 + 2^24 q3)
+      const W3 e = sub(p1, p3), z = add(mul_2_72(q1), mul_2_24(q3));
+      out[1] = reduce(sub(e, z));
+      out[5] = reduce(add(e, z));
+    }
+    {
+      // 2^-72 (q1 + 2^48 q3) = -2^24 (q1 + 2^48 q3) = -(2^24 q1 + 2^72 q3)
+      const W3 e = add(p1, p3), z = add(mul_2_24(q1), mul_2_72(q3));
+      out[3] = reduce(sub(e, z));
+      out[7] = reduce(add(e, z));
+    }
+  } else {
+    W3 h[8];
+    uint64_t lo[8], hi[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h[k] = x[k];
+    dit_inv<8>(h, lo);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h[k] = x[8 + k];
+    dit_inv<8>(h, hi);
+    // last stage: inverse twiddles 2^-12k = -2^(96 - 12 k)
+    const W3 t[8] = {from_word(shl_c<0>(hi[0])),  from_word(shl_c<84>(hi[1])), from_word(shl_c<72>(hi[2])),
+                     from_word(shl_c<60>(hi[3])), from_word(shl_c<48>(hi[4])), from_word(shl_c<36>(hi[5])),
+                     from_word(shl_c<24>(hi[6])), from_word(shl_c<12>(hi[7]))};
+    out[0] = reduce(add(from_word(lo[0]), t[0]));
+    out[8] = reduce(add_bias(sub(from_word(lo[0]), t[0])));
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+      out[k] = fold(sub(from_word(lo[k]), t[k]));
+      out[k + 8] = fold(add(from_word(lo[k]), t[k]));
+    }
+  }
+}
+
+}  // namespace lazy
+}  // namespace lnt

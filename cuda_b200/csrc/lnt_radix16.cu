@@ -66,15 +66,16 @@ __device__ __forceinline__ void row_dif_tasks(uint64_t* sm, int ld, int rows, in
     const int off = b * span + t, b0 = sw(off);
     uint64_t* base = sm + g * ld;
     uint64_t v[R];
+    lazy::W3 y[R];
     if (first) {
       const size_t rb = (size_t)g * L + off;
 #pragma unroll
-      for (int d = 0; d < R; ++d) v[d] = gl::mul(x[rb + q * d], twf[rb + q * d]);
+      for (int d = 0; d < R; ++d) y[d] = lazy::mul3(x[rb + q * d], twf[rb + q * d]);
     } else {
 #pragma unroll
-      for (int d = 0; d < R; ++d) v[d] = base[task_pos<Big>(b0, q, qs, d)];
+      for (int d = 0; d < R; ++d) y[d] = lazy::from_word(base[task_pos<Big>(b0, q, qs, d)]);
     }
-    dif<R>(v);
+    lazy::dif<R>(y, v);
     if (q > 1) mul_task_twiddles<R>(v, twL + t * R);
 #pragma unroll
     for (int r = 0; r < R; ++r) base[task_pos<Big>(b0, q, qs, r)] = v[r];
@@ -96,12 +97,16 @@ __device__ __forceinline__ void row_dit_tasks(uint64_t* sm, int ld, int rows, in
     uint64_t v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = base[task_pos<Big>(b0, q, qs, r)];
-    if (q > 1) mul_task_twiddles<R>(v, itwL + t * R);
-    dit_inv<R>(v);
+    lazy::W3 y[R];
+    if (q > 1)
+      mul_task_twiddles<R>(v, itwL + t * R, y);
+    else
+      widen<R>(v, y);
+    lazy::dit_inv<R>(y, v);
     if (last) {
       const size_t rb = (size_t)g * L + off;
 #pragma unroll
-      for (int d = 0; d < R; ++d) x[rb + q * d] = gl::mul(v[d], twi[rb + q * d]);
+      for (int d = 0; d < R; ++d) x[rb + q * d] = lazy::mul(v[d], twi[rb + q * d]);
     } else {
 #pragma unroll
       for (int d = 0; d < R; ++d) base[task_pos<Big>(b0, q, qs, d)] = v[d];
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(TH) row5_r16(const TwoPassDesc* __restrict__ D
       const int i0 = g * W + c;
       const uint64_t* base = sm + 5 * g * ld + sw(c);
       uint64_t u[5];
-      u[0] = base[0];
+      u[0] = gl::canon(base[0]);
 #pragma unroll
       for (int k5 = 1; k5 < 5; ++k5) u[k5] = gl::mul(base[k5 * ld], D.itw5[(k5 - 1) * L + c]);
       dft5(u, c5);

@@ -2,7 +2,7 @@
 //
 // The kernels reduce modulo p = 2^64 - 2^32 + 1 with PTX carry chains and
 // multiplier-pipe sums (goldilocks.cuh reduce_words / reduce_words3, the shift
-// twiddles of ntt_core.cuh).  Some of their branches are rare on residue data:
+// twiddles of ntt_core.cuh, the three-word transforms of lazy_core.cuh).  Some of their branches are rare on residue data:
 // a word >= p before the canonical step, a carry and a borrow in the same
 // reduction, a digit product whose fold carries.  Random residues reach each
 // about once in 2^32 operations.  This entry point runs the device functions
@@ -20,17 +20,35 @@
 
 #include "../../include/lucasntt.h"
 #include "goldilocks.cuh"
+#include "lazy_core.cuh"
 #include "lnt_internal.h"
 #include "ntt_core.cuh"
 
 namespace {
 
-// results per operand pair: mul, add, sub, ten shifts, three digit products
-constexpr int kOps = 16;
+// results per operand pair: mul, add, sub, ten shifts, three digit products, and the lazily
+// reduced product and transforms of 2, 4, 8 and 16 points both ways (canonicalised)
+constexpr int kLazy = 16;
+constexpr int kOps = kLazy + 1 + 2 * (2 + 4 + 8 + 16);
 
 template <unsigned S>
 __host__ __device__ uint64_t shift_op(uint64_t x) {
   return lnt::shl_c<S>(x);
+}
+
+// Forward, on words, and back, on products: positions hold a, b and words made of both that
+// sit at the ends of the 64-bit range.
+template <int R>
+__host__ __device__ void lazy_transforms(uint64_t a, uint64_t b, uint64_t* r) {
+  const uint64_t v[5] = {a, ~b, b, ~a, a ^ (b << 32)};
+  lnt::lazy::W3 x[R];
+  uint64_t out[R];
+  for (int i = 0; i < R; ++i) x[i] = lnt::lazy::from_word(v[i % 5]);
+  lnt::lazy::dif<R>(x, out);
+  for (int i = 0; i < R; ++i) r[i] = gl::canon(out[i]);
+  for (int i = 0; i < R; ++i) x[i] = lnt::lazy::mul3(v[i % 5], v[(i + 2) % 5]);
+  lnt::lazy::dit_inv<R>(x, out);
+  for (int i = 0; i < R; ++i) r[R + i] = gl::canon(out[i]);
 }
 
 __host__ __device__ void arith_ops(uint64_t a, uint64_t b, uint64_t* r) {
@@ -52,6 +70,12 @@ __host__ __device__ void arith_ops(uint64_t a, uint64_t b, uint64_t* r) {
   r[13] = gl::mul_digit((int64_t)(int32_t)b0, a);
   r[14] = gl::mul_digit((int64_t)b0, a);
   r[15] = gl::mul_digit(-(int64_t)b0, a);
+  r += kLazy;
+  *r++ = gl::canon(lnt::lazy::mul(~a, ~b));
+  lazy_transforms<2>(a, b, r);
+  lazy_transforms<4>(a, b, r + 4);
+  lazy_transforms<8>(a, b, r + 12);
+  lazy_transforms<16>(a, b, r + 28);
 }
 
 __global__ void arith_selftest_kernel(const uint64_t* a, const uint64_t* b, uint32_t count,
@@ -179,7 +203,7 @@ extern "C" int lnt_arith_selftest(int device, uint64_t* checked, uint64_t* misma
         }
       }
   }
-  *checked = (uint64_t)n * kOps;
+  *checked = (uint64_t)n * kLazy;  // the modular operations; the transforms' outputs only count when wrong
   *mismatches = bad;
   if (bad) {
     lnt::set_last_error("lnt_arith_selftest: " + std::to_string(bad) + " mismatches; first: " + first);

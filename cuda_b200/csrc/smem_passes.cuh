@@ -20,7 +20,7 @@
 #include <stdint.h>
 
 #include "goldilocks.cuh"
-#include "ntt_core.cuh"
+#include "lazy_core.cuh"
 
 namespace lnt {
 namespace smem {
@@ -62,19 +62,40 @@ __host__ __device__ inline Passes make_passes(int log2L, int b = kDefaultRadixLo
 // R/2 vector loads from one base address.  Element 0's twiddle is
 // omega^(t brev(0)) = 1 in every task: it is loaded (the vector load) but not
 // multiplied.
-#ifndef LNT_TW_UNROLL
-#define LNT_TW_UNROLL 8  // twiddle vectors loaded per unrolled step (register pressure)
-#endif
-constexpr int kTwUnroll = LNT_TW_UNROLL;
 template <int R>
-__device__ __forceinline__ void mul_task_twiddles(uint64_t (&v)[R], const uint64_t* tw) {
+__device__ __forceinline__ void load_task_twiddles(uint64_t (&w)[R], const uint64_t* tw) {
   const ulonglong2* w2 = reinterpret_cast<const ulonglong2*>(tw);
-#pragma unroll kTwUnroll
+#pragma unroll
   for (int k = 0; k < R / 2; ++k) {
     const ulonglong2 u = __ldg(w2 + k);
-    if (k > 0) v[2 * k] = gl::mul(v[2 * k], u.x);
-    v[2 * k + 1] = gl::mul(v[2 * k + 1], u.y);
+    w[2 * k] = u.x;
+    w[2 * k + 1] = u.y;
   }
+}
+
+// after a forward transform: words (any representative) times the twiddles
+template <int R>
+__device__ __forceinline__ void mul_task_twiddles(uint64_t (&v)[R], const uint64_t* tw) {
+  uint64_t w[R];
+  load_task_twiddles<R>(w, tw);
+#pragma unroll
+  for (int r = 1; r < R; ++r) v[r] = lazy::mul(v[r], w[r]);
+}
+
+// before an inverse transform: the products stay three words (lazy::mul3)
+template <int R>
+__device__ __forceinline__ void mul_task_twiddles(const uint64_t (&v)[R], const uint64_t* tw, lazy::W3 (&x)[R]) {
+  uint64_t w[R];
+  load_task_twiddles<R>(w, tw);
+  x[0] = lazy::from_word(v[0]);
+#pragma unroll
+  for (int r = 1; r < R; ++r) x[r] = lazy::mul3(v[r], w[r]);
+}
+
+template <int R>
+__device__ __forceinline__ void widen(const uint64_t (&v)[R], lazy::W3 (&x)[R]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) x[r] = lazy::from_word(v[r]);
 }
 
 // Shared-memory position of element d (d < R) of a task whose first element is
@@ -98,7 +119,9 @@ __device__ __forceinline__ void task_dif(uint64_t* base, int b0, int q, int qs, 
   uint64_t v[R];
 #pragma unroll
   for (int d = 0; d < R; ++d) v[d] = base[task_pos<Big>(b0, q, qs, d)];
-  dif<R>(v);
+  lazy::W3 x[R];
+  widen<R>(v, x);
+  lazy::dif<R>(x, v);
   if (q > 1) mul_task_twiddles<R>(v, tw);
 #pragma unroll
   for (int r = 0; r < R; ++r) base[task_pos<Big>(b0, q, qs, r)] = v[r];
@@ -110,8 +133,12 @@ __device__ __forceinline__ void task_dit(uint64_t* base, int b0, int q, int qs, 
   uint64_t v[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) v[r] = base[task_pos<Big>(b0, q, qs, r)];
-  if (q > 1) mul_task_twiddles<R>(v, itw);
-  dit_inv<R>(v);
+  lazy::W3 x[R];
+  if (q > 1)
+    mul_task_twiddles<R>(v, itw, x);
+  else
+    widen<R>(v, x);
+  lazy::dit_inv<R>(x, v);
 #pragma unroll
   for (int d = 0; d < R; ++d) base[task_pos<Big>(b0, q, qs, d)] = v[d];
 }
@@ -134,10 +161,12 @@ __device__ __forceinline__ void task_square(uint64_t* base, int off) {
   uint64_t v[R];
 #pragma unroll
   for (int d = 0; d < R; ++d) v[d] = p[d];
-  dif<R>(v);
+  lazy::W3 x[R];
+  widen<R>(v, x);
+  lazy::dif<R>(x, v);
 #pragma unroll
-  for (int d = 0; d < R; ++d) v[d] = gl::sqr(v[d]);
-  dit_inv<R>(v);
+  for (int d = 0; d < R; ++d) x[d] = lazy::mul3(v[d], v[d]);
+  lazy::dit_inv<R>(x, v);
 #pragma unroll
   for (int d = 0; d < R; ++d) p[d] = v[d];
 }
@@ -150,10 +179,12 @@ __device__ __forceinline__ void task_mul(uint64_t* base, int off, const uint64_t
   uint64_t v[R];
 #pragma unroll
   for (int d = 0; d < R; ++d) v[d] = p[d];
-  dif<R>(v);
+  lazy::W3 x[R];
+  widen<R>(v, x);
+  lazy::dif<R>(x, v);
 #pragma unroll
-  for (int d = 0; d < R; ++d) v[d] = gl::mul(v[d], f[off + d]);
-  dit_inv<R>(v);
+  for (int d = 0; d < R; ++d) x[d] = lazy::mul3(v[d], f[off + d]);
+  lazy::dit_inv<R>(x, v);
 #pragma unroll
   for (int d = 0; d < R; ++d) p[d] = v[d];
 }

@@ -1,0 +1,75 @@
+// Host check of the lazily reduced transforms (cuda_b200/csrc/lazy_core.cuh): dif<R> and
+// dit_inv<R> on any 64-bit words, and on products of such words, are congruent to the
+// canonical transforms (ntt_core.cuh) of the residues, and no intermediate leaves the ranges
+// that the three-word form assumes (lazy::range_error).  Extreme words sit at every position.
+#include <cstdint>
+#include <cstdio>
+#include <random>
+#include "../../cuda_b200/csrc/lazy_core.cuh"
+
+using namespace lnt;
+static int fails = 0;
+static uint64_t canon(uint64_t x) { return x >= gl::P ? x - gl::P : x; }
+
+static uint64_t pick(std::mt19937_64& rng) {
+  static const uint64_t edge[] = {0ull, 1ull, 0xFFFFFFFFull, 0x100000000ull, 0x8000000000000000ull, gl::P - 1,
+                                  gl::P, gl::P + 1, 0xFFFFFFFFFFFFFFFEull, 0xFFFFFFFFFFFFFFFFull};
+  const uint64_t r = rng();
+  return (r & 3) ? edge[(r >> 8) % 10] : rng();
+}
+
+template <int R>
+void check(std::mt19937_64& rng) {
+  for (int rep = 0; rep < 20000; ++rep) {
+    lazy::W3 x[R];
+    uint64_t want[R], got[R];
+    const int mode = rep % 4;  // words of all extremes, products, one extreme value everywhere, +- halves
+    const uint64_t all = pick(rng), other = pick(rng);
+    for (int i = 0; i < R; ++i) {
+      uint64_t a = mode == 2 ? all : (mode == 3 ? ((rng() & 1) ? all : other) : pick(rng));
+      if (mode == 1) {
+        const uint64_t b = pick(rng);
+        x[i] = lazy::mul3(a, b);
+        want[i] = gl::mul(canon(a), canon(b));
+        if (canon(lazy::mul(a, b)) != want[i] && fails++ < 5) std::printf("mul\n");
+      } else {
+        x[i] = lazy::from_word(a);
+        want[i] = canon(a);
+      }
+    }
+    lazy::W3 y[R];
+    uint64_t inv[R];
+    for (int i = 0; i < R; ++i) {
+      y[i] = x[i];
+      inv[i] = want[i];
+    }
+    lazy::dif<R>(x, got);
+    dif<R>(want);
+    for (int i = 0; i < R; ++i)
+      if (canon(got[i]) != want[i] && fails++ < 5) std::printf("dif<%d> %d mode %d\n", R, i, mode);
+    lazy::dit_inv<R>(y, got);
+    dit_inv<R>(inv);
+    for (int i = 0; i < R; ++i)
+      if (canon(got[i]) != inv[i] && fails++ < 5) std::printf("dit_inv<%d> %d mode %d\n", R, i, mode);
+    if (lazy::range_error()) {
+      std::printf("range error, R = %d mode %d\n", R, mode);
+      fails++;
+      lazy::range_error() = false;
+      return;
+    }
+  }
+}
+
+int main() {
+  std::mt19937_64 rng(11);
+  check<2>(rng);
+  check<4>(rng);
+  check<8>(rng);
+  check<16>(rng);
+  if (fails) {
+    std::printf("FAILED %d\n", fails);
+    return 1;
+  }
+  std::printf("ok\n");
+  return 0;
+}
