@@ -149,8 +149,9 @@ void power_table(uint32_t n, bool inverse, std::vector<uint64_t>& out) {
 }
 
 // Inter-pass twiddles of a length-n radix-16 transform in pass order: pass j
-// (span s, radix R, q = s / R) holds, for each task t < q, the run
-// omega_n^(t brev_R(r) n / s), r < R.  The last pass (q = 1) has none.
+// (span s, radix R, q = s / R) holds omega_n^(t brev_R(r) n / s) for each task t < q and r < R, at
+// index (r / 2) 2 q + 2 t + r % 2: the pairs of neighbouring tasks are neighbours.  The last pass
+// (q = 1) has none.
 void pass_table(uint32_t n, uint32_t max_radix, bool inverse, std::vector<uint64_t>& out) {
   uint32_t log2n = 0;
   while ((1u << log2n) < n) ++log2n;
@@ -163,12 +164,12 @@ void pass_table(uint32_t n, uint32_t max_radix, bool inverse, std::vector<uint64
     const uint32_t R = radix[j], q = span / R, scale = n / span;
     uint32_t bits = 0;
     while ((1u << bits) < R) ++bits;
-    for (uint32_t t = 0; t < q; ++t)
-      for (uint32_t r = 0; r < R; ++r) {
-        uint32_t b = 0;
-        for (uint32_t i = 0; i < bits; ++i) b |= ((r >> i) & 1u) << (bits - 1 - i);
-        out.push_back(pw[(size_t)t * b * scale]);
-      }
+    for (uint32_t i = 0; i < span; ++i) {
+      const uint32_t t = i / 2 % q, r = i / (2 * q) * 2 + i % 2;
+      uint32_t b = 0;
+      for (uint32_t k = 0; k < bits; ++k) b |= ((r >> k) & 1u) << (bits - 1 - k);
+      out.push_back(pw[(size_t)t * b * scale]);
+    }
     span /= R;
   }
   if (out.empty()) out.push_back(1);  // keep the pointer valid

@@ -126,7 +126,7 @@ struct TwoPassDesc {
   // radix-16 kernels: inter-pass twiddles of the row (1) and column (2)
   // transforms, and their inverses.  Pass j of a length-L transform (span s_j,
   // radix R_j, q_j = s_j / R_j) owns s_j words at offset s_0 + ... + s_{j-1};
-  // task t reads its R_j twiddles omega_L^(t brev(r) L / s_j) as one run.
+  // task t's twiddles omega_L^(t brev(r) L / s_j) are pairs 16 q_j bytes apart (pass_table).
   const uint64_t* itw1;
   const uint64_t* iitw1;
   const uint64_t* itw2;

@@ -76,7 +76,7 @@ __device__ __forceinline__ void row_dif_tasks(uint64_t* sm, int ld, int rows, in
       for (int d = 0; d < R; ++d) y[d] = lazy::from_word(base[task_pos<Big>(b0, q, qs, d)]);
     }
     lazy::dif<R>(y, v);
-    if (q > 1) mul_task_twiddles<R>(v, twL + t * R);
+    if (q > 1) mul_task_twiddles<R>(v, twL, t, q);
 #pragma unroll
     for (int r = 0; r < R; ++r) base[task_pos<Big>(b0, q, qs, r)] = v[r];
   }
@@ -99,7 +99,7 @@ __device__ __forceinline__ void row_dit_tasks(uint64_t* sm, int ld, int rows, in
     for (int r = 0; r < R; ++r) v[r] = base[task_pos<Big>(b0, q, qs, r)];
     lazy::W3 y[R];
     if (q > 1)
-      mul_task_twiddles<R>(v, itwL + t * R, y);
+      mul_task_twiddles<R>(v, itwL, t, q, y);
     else
       widen<R>(v, y);
     lazy::dit_inv<R>(y, v);

@@ -58,16 +58,17 @@ __host__ __device__ inline Passes make_passes(int log2L, int b = kDefaultRadixLo
 
 // ---- one task: R elements of one block, forward or inverse ----------------
 
-// The R twiddles of one task, a 16-byte aligned run of the pass table: read as
-// R/2 vector loads from one base address.  Element 0's twiddle is
-// omega^(t brev(0)) = 1 in every task: it is loaded (the vector load) but not
-// multiplied.
+// The R twiddles of task t: R/2 vector loads, pair k at 16 (k q + t) bytes of the pass's part of
+// the table, so neighbouring tasks read neighbouring vectors (with a task's R twiddles in one run, a
+// warp's loads were 64 bytes apart and took four times the L1 cycles: n = 2^26 3461 -> 3372 us a
+// squaring, 2048 8.80 -> 8.43).  Element 0's twiddle is omega^(t brev(0)) = 1 in every task: it is
+// loaded (the vector load) but not multiplied.
 template <int R>
-__device__ __forceinline__ void load_task_twiddles(uint64_t (&w)[R], const uint64_t* tw) {
-  const ulonglong2* w2 = reinterpret_cast<const ulonglong2*>(tw);
+__device__ __forceinline__ void load_task_twiddles(uint64_t (&w)[R], const uint64_t* tw, int t, int q) {
+  const ulonglong2* w2 = reinterpret_cast<const ulonglong2*>(tw) + t;
 #pragma unroll
   for (int k = 0; k < R / 2; ++k) {
-    const ulonglong2 u = __ldg(w2 + k);
+    const ulonglong2 u = __ldg(w2 + k * q);
     w[2 * k] = u.x;
     w[2 * k + 1] = u.y;
   }
@@ -75,18 +76,19 @@ __device__ __forceinline__ void load_task_twiddles(uint64_t (&w)[R], const uint6
 
 // after a forward transform: words (any representative) times the twiddles
 template <int R>
-__device__ __forceinline__ void mul_task_twiddles(uint64_t (&v)[R], const uint64_t* tw) {
+__device__ __forceinline__ void mul_task_twiddles(uint64_t (&v)[R], const uint64_t* tw, int t, int q) {
   uint64_t w[R];
-  load_task_twiddles<R>(w, tw);
+  load_task_twiddles<R>(w, tw, t, q);
 #pragma unroll
   for (int r = 1; r < R; ++r) v[r] = lazy::mul(v[r], w[r]);
 }
 
 // before an inverse transform: the products stay three words (lazy::mul3)
 template <int R>
-__device__ __forceinline__ void mul_task_twiddles(const uint64_t (&v)[R], const uint64_t* tw, lazy::W3 (&x)[R]) {
+__device__ __forceinline__ void mul_task_twiddles(const uint64_t (&v)[R], const uint64_t* tw, int t, int q,
+                                                  lazy::W3 (&x)[R]) {
   uint64_t w[R];
-  load_task_twiddles<R>(w, tw);
+  load_task_twiddles<R>(w, tw, t, q);
   x[0] = lazy::from_word(v[0]);
 #pragma unroll
   for (int r = 1; r < R; ++r) x[r] = lazy::mul3(v[r], w[r]);
@@ -115,27 +117,27 @@ __device__ __forceinline__ int task_pos(int b0, int q, int qs, int d) {
 
 // forward: DIF, then omega_span^(t k) (tw: this task's twiddles; unused when q == 1)
 template <int R, bool Big>
-__device__ __forceinline__ void task_dif(uint64_t* base, int b0, int q, int qs, const uint64_t* tw) {
+__device__ __forceinline__ void task_dif(uint64_t* base, int b0, int q, int qs, const uint64_t* tw, int t) {
   uint64_t v[R];
 #pragma unroll
   for (int d = 0; d < R; ++d) v[d] = base[task_pos<Big>(b0, q, qs, d)];
   lazy::W3 x[R];
   widen<R>(v, x);
   lazy::dif<R>(x, v);
-  if (q > 1) mul_task_twiddles<R>(v, tw);
+  if (q > 1) mul_task_twiddles<R>(v, tw, t, q);
 #pragma unroll
   for (int r = 0; r < R; ++r) base[task_pos<Big>(b0, q, qs, r)] = v[r];
 }
 
 // inverse: omega_span^-(t k), then DIT
 template <int R, bool Big>
-__device__ __forceinline__ void task_dit(uint64_t* base, int b0, int q, int qs, const uint64_t* itw) {
+__device__ __forceinline__ void task_dit(uint64_t* base, int b0, int q, int qs, const uint64_t* itw, int t) {
   uint64_t v[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) v[r] = base[task_pos<Big>(b0, q, qs, r)];
   lazy::W3 x[R];
   if (q > 1)
-    mul_task_twiddles<R>(v, itw, x);
+    mul_task_twiddles<R>(v, itw, t, q, x);
   else
     widen<R>(v, x);
   lazy::dit_inv<R>(x, v);
@@ -201,9 +203,9 @@ __device__ __forceinline__ void pass_tasks(uint64_t* sm, int ld, int ntrans, int
     const int b = k >> lq, t = k & (q - 1);
     uint64_t* base = sm + g * ld;
     if constexpr (Mode == 0)
-      task_dif<R, Big>(base, sw(b * span + t), q, qs, tw + t * R);
+      task_dif<R, Big>(base, sw(b * span + t), q, qs, tw, t);
     else if constexpr (Mode == 1)
-      task_dit<R, Big>(base, sw(b * span + t), q, qs, tw + t * R);
+      task_dit<R, Big>(base, sw(b * span + t), q, qs, tw, t);
     else if constexpr (Mode == 2)
       task_square<R>(base, b * span);
     else
