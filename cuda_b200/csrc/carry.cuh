@@ -42,8 +42,21 @@ GL_HD void split_output(uint64_t c, bool unsigned_mode, unsigned w, int64_t& hi,
 // that t = k 2^w + digit.
 GL_HD int64_t balance(int64_t t, unsigned w, int64_t& k) {
   w &= 31u;  // as in split_output
+#if defined(__CUDA_ARCH__)
+  // in 32-bit words: the digit needs only the low ones, and the shift is a funnel
+  const uint32_t lo = (uint32_t)t, half = 1u << (w - 1);
+  uint32_t u0, u1;
+  asm("add.cc.u32 %0, %2, %4;\n\t"
+      "addc.u32 %1, %3, 0;"
+      : "=&r"(u0), "=r"(u1)
+      : "r"(lo), "r"((uint32_t)((uint64_t)t >> 32)), "r"(half));
+  const uint32_t k0 = __funnelshift_r(u0, u1, w);
+  k = (int64_t)(((uint64_t)(uint32_t)((int32_t)u1 >> w) << 32) | k0);
+  return (int64_t)(int32_t)(lo - (k0 << w));
+#else
   k = (t + (int64_t(1) << (w - 1))) >> w;
   return t - (k << w);
+#endif
 }
 
 // A convolution output c plus the incoming carry, as one balanced digit (the
@@ -62,7 +75,13 @@ GL_HD int64_t carry_digit(uint64_t c, bool unsigned_mode, int64_t carry, unsigne
     out = hi + q;
     return d;
   }
-  const int64_t d = balance(gl::to_signed(c) + carry, w, q);
+#if defined(__CUDA_ARCH__)
+  // outputs are below p/4 in magnitude: the top bit is the sign, and c - p = c + 2^32 - 1 mod 2^64
+  const int64_t s = (int64_t)(c + (uint32_t)((int32_t)(c >> 32) >> 31));
+#else
+  const int64_t s = gl::to_signed(c);
+#endif
+  const int64_t d = balance(s + carry, w, q);
   out = q;
   return d;
 }

@@ -241,6 +241,25 @@ GL_HD W3 mul3(uint64_t a, uint64_t b) {
 // a b as a 64-bit word (congruent, not canonical)
 GL_HD uint64_t mul(uint64_t a, uint64_t b) { return fold(mul3(a, b)); }
 
+// d w for a digit |d| < 2^32 and w in [1, p], as a 64-bit word: a 32 x 64-bit product (three
+// words), of w or of p - w for a negative digit
+GL_HD uint64_t mul_digit(int64_t d, uint64_t w) {
+#if defined(__CUDA_ARCH__)
+  const uint32_t a = (uint32_t)(d < 0 ? -d : d);
+  const uint64_t s = d < 0 ? gl::P - w : w;
+  W3 t;
+  asm("mul.lo.u32    %0, %3, %4;\n\t"
+      "mul.hi.u32    %1, %3, %4;\n\t"
+      "mad.lo.cc.u32 %1, %3, %5, %1;\n\t"
+      "madc.hi.u32   %2, %3, %5, 0;"
+      : "=&r"(t.a0), "=&r"(t.a1), "=&r"(t.a2)
+      : "r"(a), "r"((uint32_t)s), "r"((uint32_t)(s >> 32)));
+  return reduce(t);  // whose sum also holds for a2 up to 2^32 - 1: wrapped it is below 2^64 - 2^33
+#else
+  return gl::mul_digit(d, w == gl::P ? 0 : w);
+#endif
+}
+
 // ---- transforms: x (natural order, overwritten) -> out (bit-reversed order), and back ----
 
 // natural in, bit-reversed out, root 2^(192/R)

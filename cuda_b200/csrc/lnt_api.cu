@@ -50,8 +50,9 @@ struct lnt_test {
   uint64_t *itw1 = nullptr, *iitw1 = nullptr, *itw2 = nullptr, *iitw2 = nullptr;
   uint64_t *tw5 = nullptr, *itw5 = nullptr;  // n = 5 * 2^k: the radix-5 step's twiddles
   uint64_t c5[4] = {};                        // and its constants
-  uint64_t *wt = nullptr, *uwt = nullptr;
-  uint8_t* widt = nullptr;
+  // separable weights of the register-pass column kernels (TwoPassDesc)
+  ulonglong2 *rowf = nullptr, *colw = nullptr;
+  uint32_t* colf = nullptr;
   int64_t* carry = nullptr;
   uint32_t* fuse = nullptr;  // carry-fused column kernel: ticket, epoch, tile flags
   // canonical readout
@@ -120,7 +121,7 @@ void free_all(lnt_test* t) {
   free_jacobi(t);
   void* ptrs[] = {t->x, t->w, t->uw, t->widths, t->status, t->rt, t->irt, t->rdesc, t->tdesc,
                   t->twf, t->twi, t->rt1, t->irt1, t->rt2, t->irt2, t->itw1, t->iitw1,
-                  t->itw2, t->iitw2, t->tw5, t->itw5, t->wt, t->uwt, t->widt, t->carry, t->fuse, t->canon,
+                  t->itw2, t->iitw2, t->tw5, t->itw5, t->rowf, t->colw, t->colf, t->carry, t->fuse, t->canon,
                   t->blk_carry, t->blk_fn, t->blk_cin, t->cflags};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -215,9 +216,11 @@ lnt::TwoPassDesc twopass_desc(const lnt_test* t) {
   d.iitw1 = t->iitw1;
   d.itw2 = t->itw2;
   d.iitw2 = t->iitw2;
-  d.wt = t->wt;
-  d.uwt = t->uwt;
-  d.widt = t->widt;
+  d.rowf = t->rowf;
+  d.colf = t->colf;
+  d.n = t->n;
+  d.qmod = t->q % t->n;
+  d.qdiv = t->q / t->n;
   d.status = t->status;
   d.n1 = t->plan.n1;
   d.n2 = t->plan.n2;
@@ -952,14 +955,15 @@ uint64_t test_device_bytes(uint32_t n) {
   Plan plan;
   if (!make_plan(n, 0, nullptr, plan)) return 0;
   const uint64_t nb = n / canon_block_size(n);
-  uint64_t b = 8ull * n * 4 + n + 4 + nb * 10 + 4;  // x, w, uw, canon, widths, status, readout
+  uint64_t b = 16ull * n + n + 4 + nb * 10 + 4;  // x, canon, widths, status, readout
+  if (!plan.fast) b += 16ull * n;                // w, uw
   if (plan.kind == PlanKind::Resident) {
     b += 8ull * n + sizeof(ResidentDesc);  // root tables
   } else {
     // carry buffer: one word per run, at most n / 4 runs (the narrowest tile)
     b += 16ull * n + 8ull * (plan.n1 + plan.n2) + 2ull * n + sizeof(TwoPassDesc) +
          4ull * (plan.n1 + 2);  // fused-kernel flags
-    if (plan.fast) b += 16ull * (plan.n1 + plan.n2) + 17ull * n;  // inner twiddles, tile-major tables
+    if (plan.fast) b += 36ull * plan.n1 + 48ull * plan.n2;  // inner twiddles, weight factors
     if (plan.five) b += 64ull * (plan.n1 / 5);                      // radix-5 twiddles
   }
   return b;
@@ -1047,7 +1051,7 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
   lnt::word_widths(exponent, n, t->h_widths.data());
 
   const uint32_t cb = lnt::canon_block_size(n), nb = n / cb;
-  if ((e = dalloc(&t->x, n)) || (e = dalloc(&t->w, n)) || (e = dalloc(&t->uw, n)) ||
+  if ((e = dalloc(&t->x, n)) ||
       (e = dalloc(&t->widths, n)) || (e = dalloc(&t->status, 1)) || (e = dalloc(&t->canon, n)) ||
       (e = dalloc(&t->blk_carry, nb)) || (e = dalloc(&t->blk_fn, nb)) ||
       (e = dalloc(&t->blk_cin, nb)) || (e = dalloc(&t->cflags, 1)) ||
@@ -1056,7 +1060,8 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
   if ((e = cudaMemcpyAsync(t->widths, t->h_widths.data(), n, cudaMemcpyHostToDevice, t->stream)) ||
       (e = cudaMemsetAsync(t->status, 0, 4, t->stream)))
     return bail(cuda_fail(e, "upload widths"));
-  if ((e = lnt::launch_weights(exponent, n, t->w, t->uw, t->stream)))
+  if (!plan.fast && ((e = dalloc(&t->w, n)) || (e = dalloc(&t->uw, n)) ||
+                     (e = lnt::launch_weights(exponent, n, t->w, t->uw, t->stream))))
     return bail(cuda_fail(e, "weights"));
 
   int st;
@@ -1075,25 +1080,27 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
            (e = lnt::launch_five_twiddles(row_points, t->tw5, t->itw5, t->c5, t->stream))))
         return bail(cuda_fail(e, "radix-5 twiddles"));
       if ((st = upload_roots(t, plan.n2, &t->itw2, &t->iitw2, plan.radix)) != LNT_OK) return bail(st);
-      if ((e = dalloc(&t->wt, n)) || (e = dalloc(&t->uwt, n)) || (e = dalloc(&t->widt, n)) ||
-          (e = lnt::launch_tile_major(t->w, t->uw, t->widths, plan.n1, plan.n2, plan.tile, t->wt,
-                                      t->uwt, t->widt, t->stream)))
-        return bail(cuda_fail(e, "tile-major tables"));
+      if ((e = dalloc(&t->rowf, 2 * (size_t)plan.n2)) || (e = dalloc(&t->colf, plan.n1)) ||
+          (e = dalloc(&t->colw, plan.n1)) ||
+          (e = lnt::launch_weight_factors(exponent, plan.n1, plan.n2, t->rowf, t->colf, t->colw, t->stream)))
+        return bail(cuda_fail(e, "weight factors"));
     }
     if ((e = dalloc(&t->twf, n)) || (e = dalloc(&t->twi, n)) ||
         (e = dalloc(&t->carry, (size_t)plan.ntiles * plan.n2)) ||
         (e = dalloc(&t->fuse, (size_t)plan.ntiles + 2)) ||
         (e = cudaMemsetAsync(t->fuse, 0, ((size_t)plan.ntiles + 2) * 4, t->stream)))
       return bail(cuda_fail(e, "allocate twiddles"));
-    if ((e = lnt::launch_twiddles(plan.n1, plan.n2, plan.log2n2, t->twf, t->twi, t->stream)))
+    if ((e = lnt::launch_twiddles(plan.n1, plan.n2, plan.log2n2, t->colw, t->twf, t->twi, t->stream)))
       return bail(cuda_fail(e, "twiddles"));
     // the device copy of the descriptor, built once every buffer it names exists
     const lnt::TwoPassDesc hd = twopass_desc(t);
-    const void* needed[] = {hd.x, hd.carry, hd.w, hd.uw, hd.widths, hd.twf, hd.twi, hd.rt1,
+    const void* needed[] = {hd.x, hd.carry, hd.widths, hd.twf, hd.twi, hd.rt1,
                             hd.irt1, hd.rt2, hd.irt2, hd.status};
     for (const void* ptr : needed)
       if (!ptr) return bail(fail(LNT_ERR_CUDA, "internal: descriptor built before its buffers"));
-    if (plan.fast && (!hd.itw1 || !hd.iitw1 || !hd.itw2 || !hd.iitw2 || !hd.wt || !hd.uwt || !hd.widt ||
+    if (!plan.fast && (!hd.w || !hd.uw))
+      return bail(fail(LNT_ERR_CUDA, "internal: descriptor built before its buffers"));
+    if (plan.fast && (!hd.itw1 || !hd.iitw1 || !hd.itw2 || !hd.iitw2 || !hd.rowf || !hd.colf ||
                       (plan.five && (!hd.tw5 || !hd.itw5))))
       return bail(fail(LNT_ERR_CUDA, "internal: descriptor built before its buffers"));
     if ((e = dalloc(&t->tdesc, 1)) ||

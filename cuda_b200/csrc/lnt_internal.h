@@ -114,11 +114,11 @@ cudaError_t launch_resident(const ResidentDesc* d_descs, uint32_t count, uint32_
 struct TwoPassDesc {
   int64_t* x;             // n words: digits, or the column-transformed residue
   int64_t* carry;         // pending run carries, index tile * n2 + row
-  const uint64_t* w;
+  const uint64_t* w;      // weights, unweights and widths by word: radix-2 kernels only
   const uint64_t* uw;
   const uint8_t* widths;
   const uint64_t* twf;    // 4-step twiddles omega_n^(j1 * brev(row)), n2 x n1
-  const uint64_t* twi;    // their inverses
+  const uint64_t* twi;    // their inverses (register-pass plans: both times a weight factor, below)
   const uint64_t* rt1;    // row roots omega_n1^k, k < n1/2
   const uint64_t* irt1;
   const uint64_t* rt2;    // column roots omega_n2^k, k < n2/2
@@ -131,11 +131,13 @@ struct TwoPassDesc {
   const uint64_t* iitw1;
   const uint64_t* itw2;
   const uint64_t* iitw2;
-  // radix-16 column kernels: w, uw, widths in tile-major order, index
-  // (tile * n2 + row) * tile_width + column-in-tile, so a row's run is contiguous
-  const uint64_t* wt;
-  const uint64_t* uwt;
-  const uint8_t* widt;
+  // register-pass column kernels: the IBDWT weight of word j = j1 + n1 j2 is g^f with
+  // f = -q j mod n = fa[j1] + fb[j2], minus n where that wraps (g^n = 2), and its width
+  // q / n + (f < q mod n).  rowf[2 j2] = {g^fb, fb}, rowf[2 j2 + 1] = {g^-fb / n, 2 g^-fb / n};
+  // colf[j1] = fa; the column's factors g^fa / 2 and g^-fa are in twf and twi.
+  const ulonglong2* rowf;
+  const uint32_t* colf;
+  uint32_t n, qmod, qdiv;  // n, q mod n, q / n
   uint32_t* status;
   // carry-fused column kernel: [0] ticket, [1] epoch, [2 + t] flag of tile t (zeroed at creation)
   uint32_t* fuse;
@@ -186,16 +188,16 @@ cudaError_t launch_col_fused_r16(const TwoPassDesc& d, const TwoPassDesc* dd, ui
 // ------------------------------------------------------------- tables ----
 cudaError_t launch_weights(uint32_t exponent, uint32_t n, uint64_t* w, uint64_t* uw,
                            cudaStream_t s);
-cudaError_t launch_twiddles(uint32_t n1, uint32_t n2, uint32_t log2n2, uint64_t* twf,
+// colw == nullptr: plain twiddles; else colw[j1] = {g^fa / 2, g^-fa} multiplied in
+cudaError_t launch_twiddles(uint32_t n1, uint32_t n2, uint32_t log2n2, const ulonglong2* colw, uint64_t* twf,
                             uint64_t* twi, cudaStream_t s);
+// the separable weights of the register-pass column kernels (TwoPassDesc), and colw
+cudaError_t launch_weight_factors(uint32_t exponent, uint32_t n1, uint32_t n2, ulonglong2* rowf, uint32_t* colf,
+                                  ulonglong2* colw, cudaStream_t s);
 // n = 5 * 2^k rows: the radix-5 step's twiddles for planes of L points (4 L words
 // each) and its constants c5 (TwoPassDesc)
 cudaError_t launch_five_twiddles(uint32_t L, uint64_t* tw5, uint64_t* itw5, uint64_t c5[4],
                                  cudaStream_t s);
-cudaError_t launch_tile_major(const uint64_t* w, const uint64_t* uw, const uint8_t* widths,
-                              uint32_t n1, uint32_t n2, uint32_t tile, uint64_t* wt, uint64_t* uwt,
-                              uint8_t* widt, cudaStream_t s);
-
 // --------------------------------------------------- canonical readout ----
 struct CanonDesc {
   const int64_t* x;        // balanced digits

@@ -427,31 +427,28 @@ __device__ __forceinline__ void tile_store(const uint64_t* sm, int ld, int64_t* 
     x[(size_t)(idx / T) * n1 + c0 + idx % T] = (int64_t)sm[(idx % T) * ld + sw(idx / T)];
 }
 
-// A row's run of T table entries, read as 16-byte vectors (tile-major tables:
-// the run is contiguous and consecutive rows are adjacent, so a warp's loads
-// are coalesced).
+// The separable weights (TwoPassDesc).  They replace weight, unweight and width tables of one
+// entry per word (34 bytes a word and squaring of the column kernel's 66): the column factors ride
+// in the 4-step twiddles, the row factors are a table of n2 entries that stays in the L1, and a
+// word's own part is whether fa + fb wraps past n.
 template <int T>
-__device__ __forceinline__ void load_run(const uint64_t* src, uint64_t (&out)[T]) {
-  const ulonglong2* v = reinterpret_cast<const ulonglong2*>(src);
+__device__ __forceinline__ void load_colf(const TwoPassDesc& D, uint32_t t0, uint32_t (&fa)[T]) {
+  const uint4* src = reinterpret_cast<const uint4*>(D.colf + (size_t)t0 * T);
 #pragma unroll
-  for (int k = 0; k < T / 2; ++k) {
-    const ulonglong2 u = v[k];
-    out[2 * k] = u.x;
-    out[2 * k + 1] = u.y;
+  for (int k = 0; k < T / 4; ++k) {
+    const uint4 u = __ldg(src + k);
+    fa[4 * k] = u.x;
+    fa[4 * k + 1] = u.y;
+    fa[4 * k + 2] = u.z;
+    fa[4 * k + 3] = u.w;
   }
 }
 
-template <int T>
-__device__ __forceinline__ void load_widths(const uint8_t* src, unsigned (&out)[T]) {
-  if constexpr (T == 8) {
-    const uint64_t u = *reinterpret_cast<const uint64_t*>(src);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) out[c] = (unsigned)((u >> (8 * c)) & 0xFF);
-  } else {
-    const uint32_t u = *reinterpret_cast<const uint32_t*>(src);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) out[c] = (u >> (8 * c)) & 0xFF;
-  }
+// f = fa + fb mod n; returns whether the sum wrapped
+__device__ __forceinline__ bool weight_exponent(uint32_t fa, uint32_t fb, uint32_t n, uint32_t& f) {
+  const uint32_t s = fa + fb;
+  f = min(s, s - n);  // s - n wraps far above n while s < n
+  return s >= n;
 }
 
 // ---- column tile bodies: tile t0 (T columns x L rows) staged in shared memory
@@ -464,13 +461,13 @@ __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes&
                                              int ld, uint32_t t0, bool apply_carries, bool cg_carries,
                                              uint32_t& status) {
   const int L = (int)D.n2;
+  const uint32_t n = D.n, qmod = D.qmod, qdiv = D.qdiv;
+  uint32_t fa[T];
+  load_colf<T>(D, t0, fa);
   // per row: carry from the previous run, then weight (balanced digit -> field)
   for (int r = threadIdx.x; r < L; r += blockDim.x) {
     const size_t run = (size_t)t0 * L + r;
-    uint64_t w[T];
-    unsigned wd[T];
-    load_run<T>(D.wt + run * T, w);
-    load_widths<T>(D.widt + run * T, wd);
+    const ulonglong2 wf = __ldg(D.rowf + 2 * r);
     int64_t carry = 0;
     if (apply_carries) {
       const int64_t* src = D.carry + (t0 > 0 ? run - L : (size_t)(D.ntiles - 1) * L + (r ? r - 1 : L - 1));
@@ -480,10 +477,12 @@ __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes&
     for (int c = 0; c < T; ++c) {
       uint64_t& v = sm[c * ld + sw(r)];
       int64_t d = (int64_t)v;
+      uint32_t f;
+      const bool wrapped = weight_exponent(fa[c], (uint32_t)wf.y, n, f);
       if (carry != 0) {
         if (c + 1 < T) {
           int64_t q;
-          d = balance(d + carry, wd[c], q);
+          d = balance(d + carry, qdiv + (f < qmod), q);
           carry = q;
         } else {
           d += carry;
@@ -491,7 +490,8 @@ __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes&
           carry = 0;
         }
       }
-      v = gl::mul_digit(d, w[c]);
+      // g^f = (g^fa / 2) g^fb 2^(not wrapped); digits stay below 2^31 (widths are at most 30)
+      v = lazy::mul_digit(wrapped ? d : d + d, wf.x);
     }
   }
   __syncthreads();
@@ -518,17 +518,23 @@ __device__ __forceinline__ void inverse_tile(const TwoPassDesc& D, const Passes&
     pass_r<1, MR>(P.radix[j], sm, ld, T, L, span, D.iitw2 + pass_table_offset(P, L, j));
     __syncthreads();
   }
+  const uint32_t n = D.n, qmod = D.qmod, qdiv = D.qdiv;
+  uint32_t fa[T];
+  load_colf<T>(D, t0, fa);
   for (int r = threadIdx.x; r < L; r += blockDim.x) {
     const size_t run = (size_t)t0 * L + r;
-    uint64_t uw[T];
-    unsigned wd[T];
-    load_run<T>(D.uwt + run * T, uw);
-    load_widths<T>(D.widt + run * T, wd);
+    const uint32_t fb = (uint32_t)__ldg(D.rowf + 2 * r).y;
+    const ulonglong2 u = __ldg(D.rowf + 2 * r + 1);
     int64_t carry = (!D.prp && t0 == 0 && r == 0) ? -2 : 0;
 #pragma unroll
     for (int c = 0; c < T; ++c) {
       uint64_t& v = sm[c * ld + sw(r)];
-      v = (uint64_t)carry_digit(gl::mul(v, uw[c]), unsigned_mode, carry, wd[c], carry);
+      uint32_t f;
+      const bool wrapped = weight_exponent(fa[c], fb, n, f);
+      // g^-f / n = g^-fa (g^-fb / n) 2^(wrapped)
+      uint64_t y = lazy::mul(v, wrapped ? u.y : u.x);
+      if (unsigned_mode) y = gl::canon(y);
+      v = (uint64_t)carry_digit(y, unsigned_mode, carry, qdiv + (f < qmod), carry);
     }
     D.carry[run] = carry;
   }

@@ -41,38 +41,51 @@ __global__ void weights_kernel(uint32_t exponent, uint32_t n, uint64_t g, uint64
 // twf[row * n1 + j1] = omega_n^(j1 * k2) with k2 = bit-reverse(row) over log2n2
 // bits: the frequency that the forward column NTT leaves in memory row `row`.
 __global__ void twiddle_kernel(uint32_t n1, uint32_t n2, uint32_t log2n2, uint64_t root,
-                               uint64_t iroot, uint64_t* twf, uint64_t* twi) {
+                               uint64_t iroot, const ulonglong2* colw, uint64_t* twf, uint64_t* twi) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)n1 * n2) return;
   const uint32_t row = (uint32_t)(idx / n1), j1 = (uint32_t)(idx % n1);
   const uint32_t k2 = __brev(row) >> (32 - log2n2);
   const uint64_t e = (uint64_t)j1 * k2;
-  twf[idx] = gl::pow(root, e);
-  twi[idx] = gl::pow(iroot, e);
+  uint64_t f = gl::pow(root, e), i = gl::pow(iroot, e);
+  if (colw) {
+    f = gl::mul(f, colw[j1].x);
+    i = gl::mul(i, colw[j1].y);
+  }
+  twf[idx] = f;
+  twi[idx] = i;
 }
 
-// natural index j = r * n1 + t * tile + c  ->  (t * n2 + r) * tile + c
-__global__ void tile_major_kernel(const uint64_t* w, const uint64_t* uw, const uint8_t* widths,
-                                  uint32_t n1, uint32_t n2, uint32_t tile, uint64_t* wt,
-                                  uint64_t* uwt, uint8_t* widt) {
-  const size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= (size_t)n1 * n2) return;
-  const uint32_t r = (uint32_t)(j / n1), col = (uint32_t)(j % n1);
-  const uint32_t t = col / tile, c = col % tile;
-  const size_t k = ((size_t)t * n2 + r) * tile + c;
-  wt[k] = w[j];
-  uwt[k] = uw[j];
-  widt[k] = widths[j];
+// f(m) = -q m mod n for the columns (m = j1 < n1) and the rows (m = n1 j2)
+__global__ void weight_factor_kernel(uint32_t exponent, uint32_t n1, uint32_t n2, uint64_t g, uint64_t ginv,
+                                     uint64_t inv2, uint64_t inv_n, ulonglong2* rowf, uint32_t* colf,
+                                     ulonglong2* colw) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, n = n1 * n2;
+  auto neg_mod = [&](uint64_t m) {
+    const uint32_t r = (uint32_t)((uint64_t)exponent * m % n);
+    return r ? n - r : 0u;
+  };
+  if (i < n1) {
+    const uint32_t f = neg_mod(i);
+    colf[i] = f;
+    colw[i] = make_ulonglong2(gl::mul(gl::pow(g, f), inv2), gl::pow(ginv, f));
+  }
+  if (i < n2) {
+    const uint32_t f = neg_mod((uint64_t)n1 * i);
+    const uint64_t u = gl::mul(gl::pow(ginv, f), inv_n);
+    rowf[2 * i] = make_ulonglong2(gl::pow(g, f), f);
+    rowf[2 * i + 1] = make_ulonglong2(u, gl::add(u, u));
+  }
 }
 
 }  // namespace
 
-cudaError_t launch_tile_major(const uint64_t* w, const uint64_t* uw, const uint8_t* widths,
-                              uint32_t n1, uint32_t n2, uint32_t tile, uint64_t* wt, uint64_t* uwt,
-                              uint8_t* widt, cudaStream_t s) {
-  const uint64_t n = (uint64_t)n1 * n2;
-  tile_major_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, uw, widths, n1, n2, tile, wt, uwt,
-                                                                 widt);
+cudaError_t launch_weight_factors(uint32_t exponent, uint32_t n1, uint32_t n2, ulonglong2* rowf, uint32_t* colf,
+                                  ulonglong2* colw, cudaStream_t s) {
+  const uint32_t n = n1 * n2, m = n1 > n2 ? n1 : n2;
+  const uint64_t g = gl::pow(7, ((gl::P - 1) / 192 / n) * 5ull);  // g^n = 2
+  weight_factor_kernel<<<(m + 127) / 128, 128, 0, s>>>(exponent, n1, n2, g, gl::inv(g), gl::inv(2), gl::inv(n),
+                                                       rowf, colf, colw);
   return cudaGetLastError();
 }
 
@@ -113,14 +126,14 @@ cudaError_t launch_five_twiddles(uint32_t L, uint64_t* tw5, uint64_t* itw5, uint
   return cudaGetLastError();
 }
 
-cudaError_t launch_twiddles(uint32_t n1, uint32_t n2, uint32_t log2n2, uint64_t* twf,
+cudaError_t launch_twiddles(uint32_t n1, uint32_t n2, uint32_t log2n2, const ulonglong2* colw, uint64_t* twf,
                             uint64_t* twi, cudaStream_t s) {
   const uint64_t n = (uint64_t)n1 * n2;
   const uint64_t root = gl::pow(554, (gl::P - 1) / n);
   const uint64_t iroot = gl::inv(root);
   const uint32_t threads = 256;
   const uint64_t blocks = (n + threads - 1) / threads;
-  twiddle_kernel<<<(unsigned)blocks, threads, 0, s>>>(n1, n2, log2n2, root, iroot, twf, twi);
+  twiddle_kernel<<<(unsigned)blocks, threads, 0, s>>>(n1, n2, log2n2, root, iroot, colw, twf, twi);
   return cudaGetLastError();
 }
 
