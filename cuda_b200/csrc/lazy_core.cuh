@@ -392,5 +392,49 @@ GL_HD void dit_inv(W3 (&x)[R], uint64_t (&out)[R]) {
   }
 }
 
+// x 4, |x| < 2^93
+GL_HD W3 mul_4(const W3& x) {
+#if defined(__CUDA_ARCH__)
+  return {x.a0 << 2, __funnelshift_l(x.a0, x.a1, 2), __funnelshift_l(x.a1, x.a2, 2)};
+#else
+  return from_int(to_int(x) * 4);
+#endif
+}
+
+// Constants of dft5 from w = omega_5, with C1 = (w + w^4)/2, C2 = (w^2 + w^3)/2, S1 = (w - w^4)/2,
+// S2 = (w^2 - w^3)/2: {2 (C1 - C2), 4 S2, 4 (S1 - S2), 4 (S1 + S2)}.
+inline void dft5_constants(uint64_t w, uint64_t c[4]) {
+  const uint64_t half = gl::inv(2), w2 = gl::mul(w, w), w3 = gl::mul(w2, w), w4 = gl::mul(w3, w);
+  const uint64_t c1 = gl::mul(gl::add(w, w4), half), c2 = gl::mul(gl::add(w2, w3), half);
+  const uint64_t s1 = gl::mul(gl::sub(w, w4), half), s2 = gl::mul(gl::sub(w2, w3), half);
+  c[0] = gl::mul(2, gl::sub(c1, c2));
+  c[1] = gl::mul(4, s2);
+  c[2] = gl::mul(4, gl::sub(s1, s2));
+  c[3] = gl::mul(4, gl::add(s1, s2));
+}
+
+// Four times the 5-point transform, |u| < 2^66, in four general products.  With a1, b1 = u1 +- u4
+// and a2, b2 = u2 +- u3 the outputs are u0 + a1 + a2 and u0 + t +- s for (t, s) = (a1 C1 + a2 C2,
+// b1 S1 + b2 S2) and (a1 C2 + a2 C1, b1 S2 - b2 S1).  C1 + C2 = -1/2 leaves one product for both t
+// (4 t = -(a1 + a2) +- 2 (a1 - a2)(C1 - C2)), three make both s.  The inverse transform is the same
+// with outputs 1, 4 and 2, 3 exchanged; the factor 4 of each goes into the unweights.
+GL_HD void dft5(const W3 (&u)[5], const uint64_t* c, uint64_t (&out)[5]) {
+  const W3 a1 = add(u[1], u[4]), b1 = sub(u[1], u[4]);
+  const W3 a2 = add(u[2], u[3]), b2 = sub(u[2], u[3]);
+  const W3 a = add(a1, a2);
+  const W3 e = mul3(reduce(add_bias(sub(a1, a2))), c[0]);
+  const W3 m = mul3(reduce(add_bias(add(b1, b2))), c[1]);
+  const W3 s1 = add(m, mul3(reduce(add_bias(b1)), c[2]));
+  const W3 s2 = sub(m, mul3(reduce(add_bias(b2)), c[3]));
+  const W3 q = add_bias(mul_4(u[0])), p = sub(q, a);
+  out[0] = reduce(add(q, mul_4(a)));
+  const W3 p1 = add(p, e), p2 = sub(p, e);
+  out[1] = reduce(add(p1, s1));
+  out[4] = reduce(sub(p1, s1));
+  out[2] = reduce(add(p2, s2));
+  out[3] = reduce(sub(p2, s2));
+}
+constexpr uint64_t kDft5Scale = 64;  // forward 4, squared 16, inverse 4
+
 }  // namespace lazy
 }  // namespace lnt

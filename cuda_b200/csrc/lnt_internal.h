@@ -146,8 +146,7 @@ struct TwoPassDesc {
   uint32_t radix;  // largest pass radix of the row and column transforms: 8 or 16
   // n = 5 * 2^k (five != 0): n1 = 5 L and log2n1 = log2 L.  tw5[(k5 - 1) L + c] =
   // omega_{5L}^(k5 c) for plane k5 = 1..4 and plane position c, itw5 its
-  // inverse; c5 = the radix-5 constants (w + w^4)/2, (w^2 + w^3)/2, (w - w^4)/2,
-  // (w^2 - w^3)/2 of w = omega_5 = omega_{5L}^L
+  // inverse; c5 = the constants of lazy::dft5 (lazy_core.cuh)
   uint32_t five;
   const uint64_t* tw5;
   const uint64_t* itw5;

@@ -245,27 +245,8 @@ __global__ void __launch_bounds__(TH) row_mul_r16(const TwoPassDesc* __restrict_
 // 4-step twiddle as the row is loaded), a twiddle, and an L-point transform of
 // each of the five planes (the passes above, bit-reversed output), whose last
 // pass runs with the square as in row_square_r16.  The inverse runs the same
-// steps backwards and stores the row; its factor 1/5 is in the unweights (1/n).
-
-// 5-point transform with the pair form u1 w^k + u4 w^-k = a C + b S (a = u1 + u4,
-// b = u1 - u4, C = (w^k + w^-k)/2, S = (w^k - w^-k)/2; likewise u2, u3 with w^2k):
-// eight multiplications instead of sixteen.  c = {C1, C2, S1, S2}.  The inverse
-// transform (w^-1) is the same with outputs 1, 4 and 2, 3 exchanged.
-__device__ __forceinline__ void dft5(uint64_t (&u)[5], const uint64_t* c) {
-  const uint64_t a1 = gl::add(u[1], u[4]), b1 = gl::sub(u[1], u[4]);
-  const uint64_t a2 = gl::add(u[2], u[3]), b2 = gl::sub(u[2], u[3]);
-  const uint64_t t1 = gl::add(gl::mul(a1, c[0]), gl::mul(a2, c[1]));
-  const uint64_t t2 = gl::add(gl::mul(a1, c[1]), gl::mul(a2, c[0]));
-  const uint64_t s1 = gl::add(gl::mul(b1, c[2]), gl::mul(b2, c[3]));
-  const uint64_t s2 = gl::sub(gl::mul(b1, c[3]), gl::mul(b2, c[2]));
-  const uint64_t u0 = u[0];
-  u[0] = gl::add(u0, gl::add(a1, a2));
-  const uint64_t p1 = gl::add(u0, t1), p2 = gl::add(u0, t2);
-  u[1] = gl::add(p1, s1);
-  u[4] = gl::sub(p1, s1);
-  u[2] = gl::add(p2, s2);
-  u[3] = gl::sub(p2, s2);
-}
+// steps backwards and stores the row; its factor 1/5 is in the unweights (1/n), and so is 1/64
+// for the factors 4 of lazy::dft5.
 
 // Mode 0: square (a squaring), 1: forward only (the operand F of a product,
 // left in x in plane-major order), 2: product with F.  A CTA takes `rows`
@@ -286,14 +267,15 @@ __global__ void __launch_bounds__(TH) row5_r16(const TwoPassDesc* __restrict__ D
   for (int item = threadIdx.x; item < rows * L; item += TH) {
     const int g = item >> lL, c = item & (L - 1);
     const int i0 = g * W + c;
-    uint64_t u[5];
+    lazy::W3 u[5];
+    uint64_t v[5];
 #pragma unroll
-    for (int j5 = 0; j5 < 5; ++j5) u[j5] = gl::mul(x[i0 + j5 * L], twf[i0 + j5 * L]);
-    dft5(u, c5);
+    for (int j5 = 0; j5 < 5; ++j5) u[j5] = lazy::mul3(x[i0 + j5 * L], twf[i0 + j5 * L]);
+    lazy::dft5(u, c5, v);
     uint64_t* base = sm + 5 * g * ld + sw(c);
-    base[0] = u[0];
+    base[0] = v[0];
 #pragma unroll
-    for (int k5 = 1; k5 < 5; ++k5) base[k5 * ld] = gl::mul(u[k5], D.tw5[(k5 - 1) * L + c]);
+    for (int k5 = 1; k5 < 5; ++k5) base[k5 * ld] = lazy::mul(v[k5], D.tw5[(k5 - 1) * L + c]);
   }
   __syncthreads();
   int span = L;
@@ -327,16 +309,17 @@ __global__ void __launch_bounds__(TH) row5_r16(const TwoPassDesc* __restrict__ D
       const int g = item >> lL, c = item & (L - 1);
       const int i0 = g * W + c;
       const uint64_t* base = sm + 5 * g * ld + sw(c);
-      uint64_t u[5];
-      u[0] = gl::canon(base[0]);
+      lazy::W3 u[5];
+      uint64_t v[5];
+      u[0] = lazy::from_word(base[0]);
 #pragma unroll
-      for (int k5 = 1; k5 < 5; ++k5) u[k5] = gl::mul(base[k5 * ld], D.itw5[(k5 - 1) * L + c]);
-      dft5(u, c5);
-      x[i0] = gl::mul(u[0], twi[i0]);
-      x[i0 + L] = gl::mul(u[4], twi[i0 + L]);
-      x[i0 + 2 * L] = gl::mul(u[3], twi[i0 + 2 * L]);
-      x[i0 + 3 * L] = gl::mul(u[2], twi[i0 + 3 * L]);
-      x[i0 + 4 * L] = gl::mul(u[1], twi[i0 + 4 * L]);
+      for (int k5 = 1; k5 < 5; ++k5) u[k5] = lazy::mul3(base[k5 * ld], D.itw5[(k5 - 1) * L + c]);
+      lazy::dft5(u, c5, v);
+      x[i0] = lazy::mul(v[0], twi[i0]);
+      x[i0 + L] = lazy::mul(v[4], twi[i0 + L]);
+      x[i0 + 2 * L] = lazy::mul(v[3], twi[i0 + 2 * L]);
+      x[i0 + 3 * L] = lazy::mul(v[2], twi[i0 + 3 * L]);
+      x[i0 + 4 * L] = lazy::mul(v[1], twi[i0 + 4 * L]);
     }
   }
 }

@@ -11,6 +11,7 @@
 // starts where its weight says.
 #include "lnt_internal.h"
 #include "goldilocks.cuh"
+#include "lazy_core.cuh"
 
 namespace lnt {
 
@@ -84,7 +85,8 @@ cudaError_t launch_weight_factors(uint32_t exponent, uint32_t n1, uint32_t n2, u
                                   ulonglong2* colw, cudaStream_t s) {
   const uint32_t n = n1 * n2, m = n1 > n2 ? n1 : n2;
   const uint64_t g = gl::pow(7, ((gl::P - 1) / 192 / n) * 5ull);  // g^n = 2
-  weight_factor_kernel<<<(m + 127) / 128, 128, 0, s>>>(exponent, n1, n2, g, gl::inv(g), gl::inv(2), gl::inv(n),
+  const uint64_t scale = n % 5 ? n : n * lazy::kDft5Scale;
+  weight_factor_kernel<<<(m + 127) / 128, 128, 0, s>>>(exponent, n1, n2, g, gl::inv(g), gl::inv(2), gl::inv(scale),
                                                        rowf, colf, colw);
   return cudaGetLastError();
 }
@@ -116,12 +118,7 @@ cudaError_t launch_five_twiddles(uint32_t L, uint64_t* tw5, uint64_t* itw5, uint
                                  cudaStream_t s) {
   // omega_{5L} = 554^((p-1)/5L) = omega_n^n2, the same root family as every other table
   const uint64_t root = gl::pow(554, (gl::P - 1) / (5ull * L)), iroot = gl::inv(root);
-  const uint64_t w = gl::pow(root, L), half = gl::inv(2);  // omega_5
-  const uint64_t w2 = gl::mul(w, w), w3 = gl::mul(w2, w), w4 = gl::mul(w3, w);
-  c5[0] = gl::mul(gl::add(w, w4), half);
-  c5[1] = gl::mul(gl::add(w2, w3), half);
-  c5[2] = gl::mul(gl::sub(w, w4), half);
-  c5[3] = gl::mul(gl::sub(w2, w3), half);
+  lazy::dft5_constants(gl::pow(root, L), c5);
   five_twiddle_kernel<<<(4 * L + 255) / 256, 256, 0, s>>>(L, root, iroot, tw5, itw5);
   return cudaGetLastError();
 }

@@ -60,8 +60,37 @@ void check(std::mt19937_64& rng) {
   }
 }
 
+// dft5 against the definition, on words and on products
+void check5(std::mt19937_64& rng) {
+  const uint64_t w = gl::pow(554, (gl::P - 1) / 5);
+  uint64_t c[4];
+  lazy::dft5_constants(w, c);
+  for (int rep = 0; rep < 20000; ++rep) {
+    lazy::W3 u[5];
+    uint64_t v[5], got[5];
+    for (int i = 0; i < 5; ++i) {
+      const uint64_t a = pick(rng), b = pick(rng);
+      u[i] = rep & 1 ? lazy::mul3(a, b) : lazy::from_word(a);
+      v[i] = rep & 1 ? gl::mul(canon(a), canon(b)) : canon(a);
+    }
+    lazy::dft5(u, c, got);
+    for (int k = 0; k < 5; ++k) {
+      uint64_t s = 0;
+      for (int i = 0; i < 5; ++i) s = gl::add(s, gl::mul(v[i], gl::pow(w, (uint64_t)(i * k))));
+      if (canon(got[k]) != gl::mul(4, s) && fails++ < 5) std::printf("dft5 %d\n", k);
+    }
+    if (lazy::range_error()) {
+      std::printf("range error, dft5\n");
+      fails++;
+      lazy::range_error() = false;
+      return;
+    }
+  }
+}
+
 int main() {
   std::mt19937_64 rng(11);
+  check5(rng);
   check<2>(rng);
   check<4>(rng);
   check<8>(rng);
