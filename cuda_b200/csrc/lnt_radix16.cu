@@ -62,7 +62,7 @@ __device__ __forceinline__ void row_dif_tasks(uint64_t* sm, int ld, int rows, in
   const int q = span / R, per = L / R, qs = q + (q >> 4);
   const int lq = __ffs(q) - 1, lper = __ffs(per) - 1;
   for (int task = threadIdx.x; task < rows * per; task += blockDim.x) {
-    const int g = task >> lper, k = task & (per - 1), b = k >> lq, t = k & (q - 1);
+    const int g = task >> lper, k = swap_tasks<R>(task & (per - 1), q, per), b = k >> lq, t = k & (q - 1);
     const int off = b * span + t, b0 = sw(off);
     uint64_t* base = sm + g * ld;
     uint64_t v[R];
@@ -91,7 +91,7 @@ __device__ __forceinline__ void row_dit_tasks(uint64_t* sm, int ld, int rows, in
   const int q = span / R, per = L / R, qs = q + (q >> 4);
   const int lq = __ffs(q) - 1, lper = __ffs(per) - 1;
   for (int task = threadIdx.x; task < rows * per; task += blockDim.x) {
-    const int g = task >> lper, k = task & (per - 1), b = k >> lq, t = k & (q - 1);
+    const int g = task >> lper, k = swap_tasks<R>(task & (per - 1), q, per), b = k >> lq, t = k & (q - 1);
     const int off = b * span + t, b0 = sw(off);
     uint64_t* base = sm + g * ld;
     uint64_t v[R];
@@ -344,70 +344,41 @@ inline bool col_latency_mode(const TwoPassDesc& d, uint32_t count) {
 template <int TH, int MR>
 constexpr int col_min_blocks() { return (MR == 16 ? 512 : 1024) / TH > 0 ? (MR == 16 ? 512 : 1024) / TH : 1; }
 
-// column stride in words: the coalesced staging (lanes = T columns x 32/T
-// rows) then hits distinct banks
-__host__ __device__ constexpr int col_ld(int L, int T) {
-  return ((padded(L) + 15) / 16) * 16 + (T >= 16 ? 1 : 16 / T);
-}
+// words of shared memory of a tile of T columns of L words (smem::Tile)
+__host__ __device__ constexpr size_t tile_words(int L, int T) { return (size_t)T * (L + L / 8); }
 
-// HBM -> shared memory without a register round trip: every word is an
-// 8-byte cp.async, so all of a thread's loads are in flight together.
-__device__ __forceinline__ void tile_load(uint64_t* sm, int ld, const int64_t* x, int L, int T,
-                                          uint32_t n1, uint32_t c0) {
-  const int rs = blockDim.x / T;  // rows per round
-  if (blockDim.x % T == 0 && rs % 16 == 0) {
-    // fixed column per thread, rows a constant stride apart: both addresses
-    // advance by a constant (sw(r + rs) = sw(r) + rs + rs / 16)
-    const int c = threadIdx.x % T, r0 = threadIdx.x / T;
-    const int64_t* src = x + (size_t)r0 * n1 + c0 + c;
-    uint32_t dst = (uint32_t)__cvta_generic_to_shared(sm + c * ld + sw(r0));
-    const size_t src_step = (size_t)rs * n1;
-    const uint32_t dst_step = (uint32_t)(rs + rs / 16) * 8;
-    for (int r = r0; r < L; r += rs, src += src_step, dst += dst_step)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
-  } else {
-    for (int idx = threadIdx.x; idx < T * L; idx += blockDim.x) {
-      const int r = idx / T, c = idx % T;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sm + c * ld + sw(r));
-      const int64_t* src = x + (size_t)r * n1 + c0 + c;
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
-    }
+// HBM -> shared memory without a register round trip: 16-byte cp.async of two adjacent columns of a
+// row, so all of a thread's loads are in flight together.
+template <int T>
+__device__ __forceinline__ void tile_load(uint64_t* sm, const int64_t* x, int L, uint32_t n1, uint32_t c0) {
+  for (int idx = threadIdx.x; idx < T / 2 * L; idx += blockDim.x) {
+    const int r = idx / (T / 2), c = 2 * (idx % (T / 2));
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sm + pos<Tile<T>>(r) + c);
+    const int64_t* src = x + (size_t)r * n1 + c0 + c;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
 // HBM -> shared memory through L2 only (ld.global.cg): for a tile another CTA
 // of the same launch has just written.
-__device__ __forceinline__ void tile_load_cg(uint64_t* sm, int ld, const int64_t* x, int L, int T,
-                                             uint32_t n1, uint32_t c0) {
+template <int T>
+__device__ __forceinline__ void tile_load_cg(uint64_t* sm, const int64_t* x, int L, uint32_t n1, uint32_t c0) {
   for (int idx = threadIdx.x; idx < T * L; idx += blockDim.x) {
     const int r = idx / T, c = idx % T;
-    sm[c * ld + sw(r)] = (uint64_t)__ldcg(x + (size_t)r * n1 + c0 + c);
+    sm[pos<Tile<T>>(r) + c] = (uint64_t)__ldcg(x + (size_t)r * n1 + c0 + c);
   }
 }
 
-// shared memory -> HBM: as tile_load, four rounds per loop iteration so the
-// shared-memory reads overlap
-__device__ __forceinline__ void tile_store(const uint64_t* sm, int ld, int64_t* x, int L, int T,
-                                           uint32_t n1, uint32_t c0) {
-  const int rs = blockDim.x / T;
-  if (blockDim.x % T == 0 && rs % 16 == 0 && L % (4 * rs) == 0) {
-    const int c = threadIdx.x % T, r0 = threadIdx.x / T;
-    int64_t* dst = x + (size_t)r0 * n1 + c0 + c;
-    const uint64_t* src = sm + c * ld + sw(r0);
-    const size_t dst_step = (size_t)rs * n1;
-    const int src_step = rs + rs / 16;
-    for (int r = r0; r < L; r += 4 * rs, dst += 4 * dst_step, src += 4 * src_step) {
-      const uint64_t v0 = src[0], v1 = src[src_step], v2 = src[2 * src_step], v3 = src[3 * src_step];
-      dst[0] = (int64_t)v0;
-      dst[dst_step] = (int64_t)v1;
-      dst[2 * dst_step] = (int64_t)v2;
-      dst[3 * dst_step] = (int64_t)v3;
-    }
-    return;
+// shared memory -> HBM, 16 bytes a thread
+template <int T>
+__device__ __forceinline__ void tile_store(const uint64_t* sm, int64_t* x, int L, uint32_t n1, uint32_t c0) {
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < T / 2 * L; idx += blockDim.x) {
+    const int r = idx / (T / 2), c = 2 * (idx % (T / 2));
+    *reinterpret_cast<ulonglong2*>(x + (size_t)r * n1 + c0 + c) =
+        *reinterpret_cast<const ulonglong2*>(sm + pos<Tile<T>>(r) + c);
   }
-  for (int idx = threadIdx.x; idx < T * L; idx += blockDim.x)
-    x[(size_t)(idx / T) * n1 + c0 + idx % T] = (int64_t)sm[(idx % T) * ld + sw(idx / T)];
 }
 
 // The separable weights (TwoPassDesc).  They replace weight, unweight and width tables of one
@@ -427,6 +398,35 @@ __device__ __forceinline__ void load_colf(const TwoPassDesc& D, uint32_t t0, uin
   }
 }
 
+// Short columns (a row or two per thread; one test alone): touch this tile's factors while its words
+// are on their way, so that the carry steps find them in the L1.
+__device__ __forceinline__ void warm_factors(const TwoPassDesc& D, uint32_t c0) {
+  const int L = (int)D.n2;
+  if (L > 512) return;
+  uint32_t u;
+  for (int r = threadIdx.x; r < L; r += blockDim.x)
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(u) : "l"(D.rowf + 2 * r));
+  if (threadIdx.x == 0) asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(u) : "l"(D.colf + c0));
+}
+
+// A row of a tile, as 16-byte vectors.
+template <int T>
+__device__ __forceinline__ void load_row(const uint64_t* row, uint64_t (&v)[T]) {
+  const ulonglong2* src = reinterpret_cast<const ulonglong2*>(row);
+#pragma unroll
+  for (int k = 0; k < T / 2; ++k) {
+    const ulonglong2 u = src[k];
+    v[2 * k] = u.x;
+    v[2 * k + 1] = u.y;
+  }
+}
+template <int T>
+__device__ __forceinline__ void store_row(uint64_t* row, const uint64_t (&v)[T]) {
+  ulonglong2* dst = reinterpret_cast<ulonglong2*>(row);
+#pragma unroll
+  for (int k = 0; k < T / 2; ++k) dst[k] = make_ulonglong2(v[2 * k], v[2 * k + 1]);
+}
+
 // f = fa + fb mod n; returns whether the sum wrapped
 __device__ __forceinline__ bool weight_exponent(uint32_t fa, uint32_t fb, uint32_t n, uint32_t& f) {
   const uint32_t s = fa + fb;
@@ -441,7 +441,7 @@ __device__ __forceinline__ bool weight_exponent(uint32_t fa, uint32_t fb, uint32
 // (written by another CTA of the same launch).
 template <int T, int MR>
 __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes& P, uint64_t* sm,
-                                             int ld, uint32_t t0, bool apply_carries, bool cg_carries,
+                                             uint32_t t0, bool apply_carries, bool cg_carries,
                                              uint32_t& status) {
   const int L = (int)D.n2;
   const uint32_t n = D.n, qmod = D.qmod, qdiv = D.qdiv;
@@ -451,6 +451,9 @@ __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes&
   for (int r = threadIdx.x; r < L; r += blockDim.x) {
     const size_t run = (size_t)t0 * L + r;
     const ulonglong2 wf = __ldg(D.rowf + 2 * r);
+    uint64_t* row = sm + pos<Tile<T>>(r);
+    uint64_t word[T];
+    load_row<T>(row, word);
     int64_t carry = 0;
     if (apply_carries) {
       const int64_t* src = D.carry + (t0 > 0 ? run - L : (size_t)(D.ntiles - 1) * L + (r ? r - 1 : L - 1));
@@ -458,7 +461,7 @@ __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes&
     }
 #pragma unroll
     for (int c = 0; c < T; ++c) {
-      uint64_t& v = sm[c * ld + sw(r)];
+      uint64_t& v = word[c];
       int64_t d = (int64_t)v;
       uint32_t f;
       const bool wrapped = weight_exponent(fa[c], (uint32_t)wf.y, n, f);
@@ -476,16 +479,17 @@ __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes&
       // g^f = (g^fa / 2) g^fb 2^(not wrapped); digits stay below 2^31 (widths are at most 30)
       v = lazy::mul_digit(wrapped ? d : d + d, wf.x);
     }
+    store_row<T>(row, word);
   }
   __syncthreads();
   int span = L;
   for (int j = 0, seg = 0; j < P.m; ++j) {
-    pass_r<0, MR>(P.radix[j], sm, ld, T, L, span, D.itw2 + seg);
+    pass_r<0, MR, Tile<T>>(P.radix[j], sm, 0, T, L, span, D.itw2 + seg);
     __syncthreads();
     seg += span;
     span /= P.radix[j];
   }
-  tile_store(sm, ld, D.x, L, T, D.n1, t0 * T);
+  tile_store<T>(sm, D.x, L, D.n1, t0 * T);
 }
 
 // Inverse column passes, unweight, carry each row's run of T words to balanced
@@ -493,12 +497,12 @@ __device__ __forceinline__ void forward_tile(const TwoPassDesc& D, const Passes&
 // The tile's transform is in `sm`; its digits are left there.
 template <int T, int MR>
 __device__ __forceinline__ void inverse_tile(const TwoPassDesc& D, const Passes& P, uint64_t* sm,
-                                             int ld, uint32_t t0, bool unsigned_mode) {
+                                             uint32_t t0, bool unsigned_mode) {
   const int L = (int)D.n2;
   int span = 1;
   for (int j = P.m - 1; j >= 0; --j) {
     span *= P.radix[j];
-    pass_r<1, MR>(P.radix[j], sm, ld, T, L, span, D.iitw2 + pass_table_offset(P, L, j));
+    pass_r<1, MR, Tile<T>>(P.radix[j], sm, 0, T, L, span, D.iitw2 + pass_table_offset(P, L, j));
     __syncthreads();
   }
   const uint32_t n = D.n, qmod = D.qmod, qdiv = D.qdiv;
@@ -508,10 +512,13 @@ __device__ __forceinline__ void inverse_tile(const TwoPassDesc& D, const Passes&
     const size_t run = (size_t)t0 * L + r;
     const uint32_t fb = (uint32_t)__ldg(D.rowf + 2 * r).y;
     const ulonglong2 u = __ldg(D.rowf + 2 * r + 1);
+    uint64_t* row = sm + pos<Tile<T>>(r);
+    uint64_t word[T];
+    load_row<T>(row, word);
     int64_t carry = (!D.prp && t0 == 0 && r == 0) ? -2 : 0;
 #pragma unroll
     for (int c = 0; c < T; ++c) {
-      uint64_t& v = sm[c * ld + sw(r)];
+      uint64_t& v = word[c];
       uint32_t f;
       const bool wrapped = weight_exponent(fa[c], fb, n, f);
       // g^-f / n = g^-fa (g^-fb / n) 2^(wrapped)
@@ -519,6 +526,7 @@ __device__ __forceinline__ void inverse_tile(const TwoPassDesc& D, const Passes&
       if (unsigned_mode) y = gl::canon(y);
       v = (uint64_t)carry_digit(y, unsigned_mode, carry, qdiv + (f < qmod), carry);
     }
+    store_row<T>(row, word);
     D.carry[run] = carry;
   }
   __syncthreads();
@@ -529,11 +537,11 @@ __global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_forward_r16(
     const TwoPassDesc* __restrict__ Ds, Passes P, int apply_carries) {
   extern __shared__ __align__(16) uint64_t sm[];
   const TwoPassDesc& D = Ds[blockIdx.y];
-  const int ld = col_ld((int)D.n2, T);
   uint32_t status = 0;
-  tile_load(sm, ld, D.x, (int)D.n2, T, D.n1, blockIdx.x * T);
+  warm_factors(D, blockIdx.x * T);
+  tile_load<T>(sm, D.x, (int)D.n2, D.n1, blockIdx.x * T);
   __syncthreads();
-  forward_tile<T, MR>(D, P, sm, ld, blockIdx.x, apply_carries != 0, false, status);
+  forward_tile<T, MR>(D, P, sm, blockIdx.x, apply_carries != 0, false, status);
   if (status) atomicOr(D.status, status);
 }
 
@@ -542,11 +550,11 @@ __global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_inverse_r16(
     const TwoPassDesc* __restrict__ Ds, Passes P, int unsigned_mode) {
   extern __shared__ __align__(16) uint64_t sm[];
   const TwoPassDesc& D = Ds[blockIdx.y];
-  const int ld = col_ld((int)D.n2, T);
-  tile_load(sm, ld, D.x, (int)D.n2, T, D.n1, blockIdx.x * T);
+  warm_factors(D, blockIdx.x * T);
+  tile_load<T>(sm, D.x, (int)D.n2, D.n1, blockIdx.x * T);
   __syncthreads();
-  inverse_tile<T, MR>(D, P, sm, ld, blockIdx.x, unsigned_mode != 0);
-  tile_store(sm, ld, D.x, (int)D.n2, T, D.n1, blockIdx.x * T);
+  inverse_tile<T, MR>(D, P, sm, blockIdx.x, unsigned_mode != 0);
+  tile_store<T>(sm, D.x, (int)D.n2, D.n1, blockIdx.x * T);
 }
 
 // ---- carry-fused column kernel: col_inverse of one squaring and col_forward
@@ -614,7 +622,7 @@ __global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_fused_r16(
   extern __shared__ __align__(16) uint64_t sm[];
   __shared__ uint32_t s_ticket, s_epoch;
   const TwoPassDesc& D = Ds[blockIdx.y];
-  const int L = (int)D.n2, ld = col_ld(L, T);
+  const int L = (int)D.n2;
   const uint32_t n1 = D.n1, ntiles = D.ntiles, last = ntiles - 1;
   uint32_t* ctl = D.fuse;
   if (threadIdx.x == 0) {
@@ -641,22 +649,23 @@ __global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_fused_r16(
   for (int i = 0; i < ninv; ++i) {
     const bool lasttile = ticket == 0 && i == 0;
     const uint32_t tile = lasttile ? last : ticket;
-    tile_load(sm, ld, D.x, L, T, n1, tile * T);
+    warm_factors(D, tile * T);
+    tile_load<T>(sm, D.x, L, n1, tile * T);
     __syncthreads();
-    inverse_tile<T, MR>(D, P, sm, ld, tile, false);
+    inverse_tile<T, MR>(D, P, sm, tile, false);
     // the last tile's digits wait in x for the last ticket
-    if (lasttile) tile_store(sm, ld, D.x, L, T, n1, last * T);
+    if (lasttile) tile_store<T>(sm, D.x, L, n1, last * T);
     publish_flag(ctl + 2 + tile, ready);
   }
   if (is_last) {
     // the last tile's first half was done by ticket 0 (digits in x)
     wait_flag(ctl + 2 + last, ready, D.status);
-    tile_load_cg(sm, ld, D.x, L, T, n1, last * T);
+    tile_load_cg<T>(sm, D.x, L, n1, last * T);
   }
   // second half: carries in from the tile before (tile 0: the last tile, made
   // by this CTA), weight, forward column transform
   if (ticket > 0) wait_flag(ctl + 2 + ticket - 1, ready, D.status);
-  forward_tile<T, MR>(D, P, sm, ld, ticket, true, true, status);
+  forward_tile<T, MR>(D, P, sm, ticket, true, true, status);
   if (is_last && threadIdx.x == 0) {
     // every ticket of this launch is taken and every CTA has read the epoch
     ctl[0] = 0;
@@ -737,8 +746,7 @@ cudaError_t row_square_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t c
   const size_t smem = (size_t)rows * padded(L) * 8;
   cudaError_t e = ensure_smem(row_square_r16<TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  row_square_r16<TH, MR><<<dim3(d.n2 / rows, count), TH, smem, s>>>(
-      dd, make_passes((int)d.log2n1, radix_log2(d)), rows);
+  row_square_r16<TH, MR><<<dim3(d.n2 / rows, count), TH, smem, s>>>(dd, make_passes((int)d.log2n1, radix_log2(d)), rows);
   return cudaGetLastError();
 }
 
@@ -748,8 +756,7 @@ cudaError_t row_forward_t(const TwoPassDesc& d, const TwoPassDesc* dd, cudaStrea
   const size_t smem = (size_t)rows * padded(L) * 8;
   cudaError_t e = ensure_smem(row_forward_r16<TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  row_forward_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(
-      dd, make_passes((int)d.log2n1, radix_log2(d)), rows);
+  row_forward_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(dd, make_passes((int)d.log2n1, radix_log2(d)), rows);
   return cudaGetLastError();
 }
 
@@ -759,8 +766,7 @@ cudaError_t row_mul_t(const TwoPassDesc& d, const TwoPassDesc* dd, const uint64_
   const size_t smem = (size_t)rows * padded(L) * 8;
   cudaError_t e = ensure_smem(row_mul_r16<TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  row_mul_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(
-      dd, make_passes((int)d.log2n1, radix_log2(d)), rows, F);
+  row_mul_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(dd, make_passes((int)d.log2n1, radix_log2(d)), rows, F);
   return cudaGetLastError();
 }
 
@@ -858,32 +864,29 @@ cudaError_t col_dispatch(uint32_t n2, bool latency, F&& f) {
 template <int T, int TH, int MR>
 cudaError_t col_forward_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count, bool apply,
                           cudaStream_t s) {
-  const size_t smem = (size_t)T * col_ld((int)d.n2, T) * 8;
+  const size_t smem = tile_words((int)d.n2, T) * 8;
   cudaError_t e = ensure_smem(col_forward_r16<T, TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  col_forward_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(
-      dd, make_passes((int)d.log2n2, radix_log2(d)), apply ? 1 : 0);
+  col_forward_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, radix_log2(d)), apply ? 1 : 0);
   return cudaGetLastError();
 }
 
 template <int T, int TH, int MR>
 cudaError_t col_inverse_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count,
                           bool unsigned_mode, cudaStream_t s) {
-  const size_t smem = (size_t)T * col_ld((int)d.n2, T) * 8;
+  const size_t smem = tile_words((int)d.n2, T) * 8;
   cudaError_t e = ensure_smem(col_inverse_r16<T, TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  col_inverse_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(
-      dd, make_passes((int)d.log2n2, radix_log2(d)), unsigned_mode ? 1 : 0);
+  col_inverse_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, radix_log2(d)), unsigned_mode ? 1 : 0);
   return cudaGetLastError();
 }
 
 template <int T, int TH, int MR>
 cudaError_t col_fused_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count, cudaStream_t s) {
-  const size_t smem = (size_t)T * col_ld((int)d.n2, T) * 8;
+  const size_t smem = tile_words((int)d.n2, T) * 8;
   cudaError_t e = ensure_smem(col_fused_r16<T, TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  col_fused_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(
-      dd, make_passes((int)d.log2n2, radix_log2(d)));
+  col_fused_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, radix_log2(d)));
   return cudaGetLastError();
 }
 

@@ -28,6 +28,23 @@ namespace smem {
 __host__ __device__ __forceinline__ int sw(int i) { return i + (i >> 4); }
 __host__ __device__ constexpr int padded(int L) { return L + L / 16; }
 
+// Where element i of transform g lies.  Rows: the transforms one after another (ld words apart),
+// one word of padding in 16.  Tile<T>: T transforms interleaved, word (i, g) at T (i + i / 8) + g, so a
+// row of T words stays together: it is copied 16 bytes at a time, read as vectors by the carry
+// steps, and T neighbouring threads share their twiddles.  Both layouts keep off + q d at a
+// constant stride in d (q >= 16, or 8 for Tile) and every pass free of bank conflicts.
+struct Rows {
+  static constexpr int kStride = 1, kPadLog2 = 4, kTile = 1;
+};
+template <int T>
+struct Tile {
+  static constexpr int kStride = T, kPadLog2 = 3, kTile = T;
+};
+template <class Lay>
+__host__ __device__ __forceinline__ int pos(int i) {
+  return Lay::kStride * (i + (i >> Lay::kPadLog2));
+}
+
 struct Passes {
   int m;          // number of passes
   int radix[6];   // r_0 (largest stride) ... r_{m-1} (contiguous)
@@ -105,36 +122,45 @@ __device__ __forceinline__ void widen(const uint64_t (&v)[R], lazy::W3 (&x)[R]) 
 // sw(off + q d) = sw(off) + q d + (q d >> 4), because the low four bits of
 // off + q d never carry out of a padding group of 16 words.  For q >= 16 that
 // is sw(off) + d (q + q / 16): one stride per pass, no per-element index math.
-template <bool Big>
+template <bool Big, class Lay = Rows>
 __device__ __forceinline__ int task_pos(int b0, int q, int qs, int d) {
   if constexpr (Big) {
     return b0 + d * qs;
   } else {
-    const int k = q * d;
-    return b0 + k + (k >> 4);
+    return b0 + pos<Lay>(q * d);
   }
 }
 
+// Which task of a pass a thread takes.  With q = 8 the 16 threads of a shared-memory access would
+// take two neighbouring blocks of 64 words, 68 words apart in the padded layout: half of their banks
+// collide.  Exchanging the two low bits of the block number puts blocks 136 words apart together,
+// whose banks do not.
+template <int R, class Lay = Rows>
+__device__ __forceinline__ int swap_tasks(int k, int q, int per) {
+  if (Lay::kTile == 1 && R == 8 && q == 8 && per >= 32) return (k & ~24) | ((k & 8) << 1) | ((k >> 1) & 8);
+  return k;
+}
+
 // forward: DIF, then omega_span^(t k) (tw: this task's twiddles; unused when q == 1)
-template <int R, bool Big>
+template <int R, bool Big, class Lay>
 __device__ __forceinline__ void task_dif(uint64_t* base, int b0, int q, int qs, const uint64_t* tw, int t) {
   uint64_t v[R];
 #pragma unroll
-  for (int d = 0; d < R; ++d) v[d] = base[task_pos<Big>(b0, q, qs, d)];
+  for (int d = 0; d < R; ++d) v[d] = base[task_pos<Big, Lay>(b0, q, qs, d)];
   lazy::W3 x[R];
   widen<R>(v, x);
   lazy::dif<R>(x, v);
   if (q > 1) mul_task_twiddles<R>(v, tw, t, q);
 #pragma unroll
-  for (int r = 0; r < R; ++r) base[task_pos<Big>(b0, q, qs, r)] = v[r];
+  for (int r = 0; r < R; ++r) base[task_pos<Big, Lay>(b0, q, qs, r)] = v[r];
 }
 
 // inverse: omega_span^-(t k), then DIT
-template <int R, bool Big>
+template <int R, bool Big, class Lay>
 __device__ __forceinline__ void task_dit(uint64_t* base, int b0, int q, int qs, const uint64_t* itw, int t) {
   uint64_t v[R];
 #pragma unroll
-  for (int r = 0; r < R; ++r) v[r] = base[task_pos<Big>(b0, q, qs, r)];
+  for (int r = 0; r < R; ++r) v[r] = base[task_pos<Big, Lay>(b0, q, qs, r)];
   lazy::W3 x[R];
   if (q > 1)
     mul_task_twiddles<R>(v, itw, t, q, x);
@@ -142,7 +168,7 @@ __device__ __forceinline__ void task_dit(uint64_t* base, int b0, int q, int qs, 
     widen<R>(v, x);
   lazy::dit_inv<R>(x, v);
 #pragma unroll
-  for (int d = 0; d < R; ++d) base[task_pos<Big>(b0, q, qs, d)] = v[d];
+  for (int d = 0; d < R; ++d) base[task_pos<Big, Lay>(b0, q, qs, d)] = v[d];
 }
 
 // Offset of pass j's twiddles in a pass table (the spans of the passes before it).
@@ -191,21 +217,22 @@ __device__ __forceinline__ void task_mul(uint64_t* base, int off, const uint64_t
   for (int d = 0; d < R; ++d) p[d] = v[d];
 }
 
-template <int R, int Mode, bool Big>
+template <int R, int Mode, bool Big, class Lay>
 __device__ __forceinline__ void pass_tasks(uint64_t* sm, int ld, int ntrans, int L, int span,
                                            const uint64_t* tw) {
   // all sizes are powers of two: index arithmetic by shifts and masks
-  const int q = span / R, per = L / R, qs = q + (q >> 4);
+  const int q = span / R, per = L / R, qs = pos<Lay>(q);
   const int lq = __ffs(q) - 1, lper = __ffs(per) - 1;
-  const int total = ntrans * per;
+  const int total = (Lay::kTile > 1 ? Lay::kTile : ntrans) * per;
   for (int task = threadIdx.x; task < total; task += blockDim.x) {
-    const int g = task >> lper, k = task & (per - 1);
+    const int g = Lay::kTile > 1 ? task & (Lay::kTile - 1) : task >> lper;
+    const int k = swap_tasks<R, Lay>(Lay::kTile > 1 ? task / Lay::kTile : task & (per - 1), q, per);
     const int b = k >> lq, t = k & (q - 1);
-    uint64_t* base = sm + g * ld;
+    uint64_t* base = Lay::kTile > 1 ? sm + g : sm + g * ld;
     if constexpr (Mode == 0)
-      task_dif<R, Big>(base, sw(b * span + t), q, qs, tw, t);
+      task_dif<R, Big, Lay>(base, pos<Lay>(b * span + t), q, qs, tw, t);
     else if constexpr (Mode == 1)
-      task_dit<R, Big>(base, sw(b * span + t), q, qs, tw, t);
+      task_dit<R, Big, Lay>(base, pos<Lay>(b * span + t), q, qs, tw, t);
     else if constexpr (Mode == 2)
       task_square<R>(base, b * span);
     else
@@ -213,27 +240,27 @@ __device__ __forceinline__ void pass_tasks(uint64_t* sm, int ld, int ntrans, int
   }
 }
 
-// A pass over `ntrans` transforms of length L; transform g lives at sm + g * ld.
+// A pass over `ntrans` transforms of length L; in the Rows layout transform g lives at sm + g * ld.
 // tw: this pass's part of the pass table.
-// Mode 0: DIF, 1: DIT, 2: square, 3: product with the transformed rows at tw
-template <int R, int Mode>
+// Mode 0: DIF, 1: DIT, 2: square, 3: product with the transformed rows at tw (Rows only)
+template <int R, int Mode, class Lay>
 __device__ void pass(uint64_t* sm, int ld, int ntrans, int L, int span, const uint64_t* tw) {
-  if (span / R >= 16)
-    pass_tasks<R, Mode, true>(sm, ld, ntrans, L, span, tw);
+  if (span / R >= (1 << Lay::kPadLog2))
+    pass_tasks<R, Mode, true, Lay>(sm, ld, ntrans, L, span, tw);
   else
-    pass_tasks<R, Mode, false>(sm, ld, ntrans, L, span, tw);
+    pass_tasks<R, Mode, false, Lay>(sm, ld, ntrans, L, span, tw);
 }
 
 // A pass of radix R (a power of two up to MR, the largest the kernel is built for).
-template <int Mode, int MR = kMaxRadix>
+template <int Mode, int MR = kMaxRadix, class Lay = Rows>
 __device__ __forceinline__ void pass_r(int R, uint64_t* sm, int ld, int ntrans, int L, int span,
                                        const uint64_t* tw) {
   switch (R) {
-    case 2: pass<2, Mode>(sm, ld, ntrans, L, span, tw); break;
-    case 4: pass<4, Mode>(sm, ld, ntrans, L, span, tw); break;
-    case 8: pass<8, Mode>(sm, ld, ntrans, L, span, tw); break;
+    case 2: pass<2, Mode, Lay>(sm, ld, ntrans, L, span, tw); break;
+    case 4: pass<4, Mode, Lay>(sm, ld, ntrans, L, span, tw); break;
+    case 8: pass<8, Mode, Lay>(sm, ld, ntrans, L, span, tw); break;
     default:
-      if constexpr (MR >= 16) pass<16, Mode>(sm, ld, ntrans, L, span, tw);
+      if constexpr (MR >= 16) pass<16, Mode, Lay>(sm, ld, ntrans, L, span, tw);
       break;
   }
 }
