@@ -50,6 +50,7 @@ struct lnt_test {
   uint64_t *itw1 = nullptr, *iitw1 = nullptr, *itw2 = nullptr, *iitw2 = nullptr;
   uint64_t *tw5 = nullptr, *itw5 = nullptr;  // n = 5 * 2^k: the radix-5 step's twiddles
   uint64_t c5[4] = {};                        // and its constants
+  uint64_t* pw = nullptr;  // omega_n^e of the cluster kernel (512 ... 32768 words, policy plans)
   // separable weights of the register-pass column kernels (TwoPassDesc)
   ulonglong2 *rowf = nullptr, *colw = nullptr;
   uint32_t* colf = nullptr;
@@ -121,7 +122,7 @@ void free_all(lnt_test* t) {
   free_jacobi(t);
   void* ptrs[] = {t->x, t->w, t->uw, t->widths, t->status, t->rt, t->irt, t->rdesc, t->tdesc,
                   t->twf, t->twi, t->rt1, t->irt1, t->rt2, t->irt2, t->itw1, t->iitw1,
-                  t->itw2, t->iitw2, t->tw5, t->itw5, t->rowf, t->colw, t->colf, t->carry, t->fuse, t->canon,
+                  t->itw2, t->iitw2, t->tw5, t->itw5, t->rowf, t->colw, t->colf, t->pw, t->carry, t->fuse, t->canon,
                   t->blk_carry, t->blk_fn, t->blk_cin, t->cflags};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -428,7 +429,54 @@ void capture_graph(lnt_test* t, const lnt::TwoPassDesc& d) {
   if (!t->graph) t->graph_failed = true;
 }
 
+// Policy plans of 512 to 32768 words also run on the cluster kernel.
+bool cluster_plan(const lnt::Plan& p) {
+  return p.policy && !p.five && p.log2n >= lnt::kClusterMinLog2 && p.log2n <= lnt::kClusterMaxLog2;
+}
+
+lnt::ClusterDesc cluster_desc(const lnt_test* t, uint64_t iterations) {
+  lnt::ClusterDesc d{};
+  d.digits = t->x;
+  d.w = t->w;
+  d.uw = t->uw;
+  d.widths = t->widths;
+  d.pw = t->pw;
+  d.status = t->status;
+  d.iterations = iterations;
+  d.n = t->n;
+  d.log2n = t->plan.log2n;
+  d.prp = (uint32_t)t->prp;
+  d.unsigned_first = t->canonical_input ? 1 : 0;
+  d.short_runs = lnt::r16_run_words_needed(t->q, t->n) <= 4 ? 1 : 0;
+  if (t->plan.kind == lnt::PlanKind::TwoPass) {
+    d.colw = t->colw;
+    d.rowf = t->rowf;
+    d.colf = t->colf;
+    d.n1 = t->plan.n1;
+    d.n2 = t->plan.n2;
+    d.tile = t->plan.tile;
+    d.ntiles = t->plan.ntiles;
+    if (t->pending_carries) d.carry = t->carry;
+  }
+  return d;
+}
+
 int queue_iterations(lnt_test* t, uint64_t iterations, LaunchTimer* timer) {
+  const lnt::ClusterChoice cl = cluster_plan(t->plan) ? lnt::cluster_choice(t->n, t->n, 1) : lnt::ClusterChoice();
+  if (cl.size) {
+    const lnt::ClusterDesc d = cluster_desc(t, iterations);
+    LNT_LAUNCH(lnt::launch_cluster(nullptr, d, 1, t->n, cl.size, cl.threads, cl.pass_log2, t->stream),
+               "cluster_square_loop");
+    if (t->plan.kind == lnt::PlanKind::TwoPass && !t->pending_carries) {
+      // the two-pass kernels expect run carries from here on: none are left
+      LNT_CUDA(cudaMemsetAsync(t->carry, 0, (size_t)t->plan.ntiles * t->plan.n2 * 8, t->stream), "clear carries");
+      t->pending_carries = true;
+    }
+    t->canonical_input = false;
+    t->pristine = false;
+    t->canon_valid = false;
+    return LNT_OK;
+  }
   if (t->plan.kind == lnt::PlanKind::Resident) {
     lnt::ResidentDesc d{};
     d.digits = t->x;
@@ -942,6 +990,7 @@ ResidentDesc test_resident_desc(const lnt_test* t, uint64_t iterations) {
   d.short_runs = r16_run_words_needed(t->q, t->n) <= 4 ? 1 : 0;
   return d;
 }
+ClusterDesc test_cluster_desc(const lnt_test* t, uint64_t iterations) { return cluster_desc(t, iterations); }
 // bookkeeping after squarings were launched outside lnt_iterate
 void test_mark_iterated(lnt_test* t) {
   if (t->plan.kind == PlanKind::TwoPass) t->pending_carries = true;
@@ -957,6 +1006,7 @@ uint64_t test_device_bytes(uint32_t n) {
   const uint64_t nb = n / canon_block_size(n);
   uint64_t b = 16ull * n + n + 4 + nb * 10 + 4;  // x, canon, widths, status, readout
   if (!plan.fast) b += 16ull * n;                // w, uw
+  if (cluster_plan(plan)) b += 8ull * n;         // powers
   if (plan.kind == PlanKind::Resident) {
     b += 8ull * n + sizeof(ResidentDesc);  // root tables
   } else {
@@ -1065,6 +1115,14 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
     return bail(cuda_fail(e, "weights"));
 
   int st;
+  std::vector<uint64_t> powers;
+  if (cluster_plan(plan)) {
+    power_table(n, false, powers);
+    if ((e = dalloc(&t->pw, n)) ||
+        (e = cudaMemcpyAsync(t->pw, powers.data(), (size_t)n * 8, cudaMemcpyHostToDevice, t->stream)) ||
+        (e = cudaStreamSynchronize(t->stream)))
+      return bail(cuda_fail(e, "powers"));
+  }
   if (plan.kind == lnt::PlanKind::Resident) {
     if ((st = upload_roots(t, n, &t->rt, &t->irt, 8)) != LNT_OK) return bail(st);  // the resident kernel's passes
     if ((e = dalloc(&t->rdesc, 1))) return bail(cuda_fail(e, "allocate descriptor"));

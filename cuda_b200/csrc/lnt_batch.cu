@@ -114,6 +114,7 @@ struct lnt_batch {
   std::vector<size_t> singles;       // tests iterated one by one
   lnt::ResidentDesc* d_rdescs = nullptr;
   size_t rcap = 0;
+  lnt::ClusterDesc* d_cdescs = nullptr;  // the same tests when few enough for the cluster kernel
   std::vector<cudaStream_t> spare_streams;
   cudaStream_t rstream = nullptr;    // the resident launch, beside the groups
   cudaEvent_t fork = nullptr;        // recorded on `stream` before the group launches
@@ -294,6 +295,9 @@ int rebuild(lnt_batch* b) {
     if (b->d_rdescs) cudaFree(b->d_rdescs);
     b->rcap = std::max<size_t>(b->resident.size(), 2 * b->rcap);
     BCUDA(cudaMalloc((void**)&b->d_rdescs, b->rcap * sizeof(lnt::ResidentDesc)), "resident descriptors");
+    if (b->d_cdescs) cudaFree(b->d_cdescs);
+    b->d_cdescs = nullptr;
+    BCUDA(cudaMalloc((void**)&b->d_cdescs, b->rcap * sizeof(lnt::ClusterDesc)), "resident descriptors");
   }
   b->dirty = false;
   return LNT_OK;
@@ -373,6 +377,7 @@ int lnt_batch_destroy(lnt_batch* b) {
   for (cudaStream_t s : b->spare_streams)
     if (s) cudaStreamDestroy(s);
   if (b->d_rdescs) cudaFree(b->d_rdescs);
+  if (b->d_cdescs) cudaFree(b->d_cdescs);
   if (b->stream) cudaStreamDestroy(b->stream);
   if (b->rstream) cudaStreamDestroy(b->rstream);
   delete b;
@@ -668,21 +673,38 @@ int lnt_batch_run(lnt_batch* b, uint64_t iterations) {
   uint64_t resident_work = 0;  // word-squarings of the slowest CTA
   if (!b->resident.empty()) {
     std::vector<lnt::ResidentDesc> h;
-    uint32_t max_n = 0;
+    std::vector<lnt::ClusterDesc> hc;
+    uint32_t max_n = 0, min_n = ~0u;
     const double rate = b->resident_rate > 0 ? b->resident_rate : 5e-9;
     for (size_t i : b->resident) {
       Entry& e = b->active[i];
       if (budget)
         step[i] = std::min<uint64_t>(step[i], std::max<uint64_t>(1, (uint64_t)(b->step_seconds / (rate * e.n))));
       h.push_back(lnt::test_resident_desc(e.t, step[i]));
+      hc.push_back(lnt::test_cluster_desc(e.t, step[i]));
       max_n = std::max(max_n, e.n);
+      min_n = std::min(min_n, e.n);
       resident_work = std::max<uint64_t>(resident_work, step[i] * e.n);
     }
-    BCUDA(cudaMemcpyAsync(b->d_rdescs, h.data(), h.size() * sizeof(lnt::ResidentDesc),
-                          cudaMemcpyHostToDevice, b->rstream),
-          "upload resident descriptors");
-    BCUDA(cudaEventRecord(b->r0, b->rstream), "resident timer");
-    BCUDA(lnt::launch_resident(b->d_rdescs, (uint32_t)h.size(), max_n, b->rstream), "resident kernel");
+    // few tests: each over a cluster of CTAs; else one CTA per test
+    lnt::ClusterChoice cl;
+    if (std::all_of(hc.begin(), hc.end(), [](const lnt::ClusterDesc& d) { return d.pw != nullptr; }))
+      cl = lnt::cluster_choice(min_n, max_n, (uint32_t)h.size());
+    if (cl.size) {
+      BCUDA(cudaMemcpyAsync(b->d_cdescs, hc.data(), hc.size() * sizeof(lnt::ClusterDesc),
+                            cudaMemcpyHostToDevice, b->rstream),
+            "upload resident descriptors");
+      BCUDA(cudaEventRecord(b->r0, b->rstream), "resident timer");
+      BCUDA(lnt::launch_cluster(b->d_cdescs, hc[0], (uint32_t)hc.size(), max_n, cl.size, cl.threads, cl.pass_log2,
+                                b->rstream),
+            "cluster kernel");
+    } else {
+      BCUDA(cudaMemcpyAsync(b->d_rdescs, h.data(), h.size() * sizeof(lnt::ResidentDesc),
+                            cudaMemcpyHostToDevice, b->rstream),
+            "upload resident descriptors");
+      BCUDA(cudaEventRecord(b->r0, b->rstream), "resident timer");
+      BCUDA(lnt::launch_resident(b->d_rdescs, (uint32_t)h.size(), max_n, b->rstream), "resident kernel");
+    }
     BCUDA(cudaEventRecord(b->r1, b->rstream), "resident timer");
   }
   if (!b->groups.empty() && (st = launch_groups(b)) != LNT_OK) return st;

@@ -36,6 +36,7 @@ struct Plan {
   // the GPU (at n = 2^23: 244.6 us for the pair that takes 270.1 us as two
   // launches); below, where a squaring is latency-bound, two plain launches win
   bool fused = false;
+  bool policy = false;  // the policy's own choice (also when named explicitly): may use the cluster kernel
   // n = 5 * 2^k: rows of n1 = 5 L words, each row transform a radix-5 step over
   // the words c + L j5 followed by an L-point NTT of each of the five planes
   // (register-pass plans only; log2n1 is then log2 L)
@@ -109,6 +110,39 @@ size_t resident_smem_bytes(uint32_t n, uint32_t threads);
 uint32_t resident_threads(uint32_t n, uint32_t count, uint32_t sms);
 cudaError_t launch_resident(const ResidentDesc* d_descs, uint32_t count, uint32_t max_n,
                             cudaStream_t stream);
+
+// ------------------------------------------------------ cluster kernel ----
+// One residue over the shared memories of a thread-block cluster (lnt_cluster.cu).
+struct ClusterDesc {
+  int64_t* digits;        // n words, natural order
+  int64_t* carry;         // pending run carries of a two-pass state (cleared), or nullptr
+  const uint64_t* w;      // weights and unweights (resident tests), or nullptr:
+  const uint64_t* uw;
+  const ulonglong2* colw;  // ... the separable weights of a two-pass test (TwoPassDesc)
+  const ulonglong2* rowf;
+  const uint32_t* colf;
+  const uint8_t* widths;
+  const uint64_t* pw;     // omega_n^e, e < n
+  uint32_t* status;
+  uint64_t iterations;
+  uint32_t n, log2n, prp;
+  uint32_t unsigned_first;  // as ResidentDesc
+  uint32_t short_runs;
+  uint32_t n1, n2, tile, ntiles;  // run geometry when carry != nullptr
+};
+constexpr uint32_t kClusterMinLog2 = 9, kClusterMaxLog2 = 15;
+
+// CTAs per cluster (0: none), threads per CTA and log2 of the local passes' largest radix for
+// `count` tests of min_n to max_n words in one launch
+struct ClusterChoice {
+  uint32_t size = 0;
+  int threads = 0, pass_log2 = 3;
+};
+ClusterChoice cluster_choice(uint32_t min_n, uint32_t max_n, uint32_t count);
+bool cluster_fits(uint32_t n, uint32_t C);
+// descs == nullptr: the one test `one`
+cudaError_t launch_cluster(const ClusterDesc* descs, const ClusterDesc& one, uint32_t count, uint32_t max_n,
+                           uint32_t C, int threads, int pass_log2, cudaStream_t s);
 
 // ------------------------------------------------------ two-pass kernels ----
 struct TwoPassDesc {
@@ -233,6 +267,7 @@ const TwoPassDesc* test_twopass_device_desc(const lnt_test* t);
 TwoPassDesc test_twopass_desc(const lnt_test* t);
 bool test_ready_for_group(const lnt_test* t);
 ResidentDesc test_resident_desc(const lnt_test* t, uint64_t iterations);
+ClusterDesc test_cluster_desc(const lnt_test* t, uint64_t iterations);
 void test_mark_iterated(lnt_test* t);
 uint64_t test_device_bytes(uint32_t n);
 void set_last_error(const std::string& msg);

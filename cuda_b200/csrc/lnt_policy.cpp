@@ -186,6 +186,7 @@ bool make_plan(uint32_t n, uint32_t exponent, const PlanOptions* opt, Plan& plan
     if (o.log2_rows || o.tile || o.radix || o.fused)
       return reject("resident plan takes no split, tile, radix or fusion choice");
     plan.kind = PlanKind::Resident;
+    plan.policy = true;  // the family has no other choice
     name_plan(plan);
     return true;
   }
@@ -243,6 +244,12 @@ bool make_plan(uint32_t n, uint32_t exponent, const PlanOptions* opt, Plan& plan
     // fill the GPU; the autotuner may choose either way at any length
     plan.fused = o.fused ? o.fused == 1 : plan.log2n >= 19;
   }
+  // explicit choices that name the policy's own plan are that plan
+  Plan own;
+  const bool chosen = opt && (opt->kind || opt->log2_rows || opt->tile || opt->radix || opt->fused);
+  plan.policy = !chosen || (make_plan(n, exponent, nullptr, own) && own.fast == plan.fast &&
+                            own.log2n2 == plan.log2n2 && own.tile == plan.tile && own.radix == plan.radix &&
+                            own.fused == plan.fused);
   name_plan(plan);
   return true;
 }
