@@ -94,20 +94,26 @@ GL_HD W3 add_bias(const W3& x) {
 __device__ __forceinline__ uint32_t sign_word(uint32_t a2) { return (uint32_t)((int32_t)a2 >> 31); }
 #endif
 
-// x 2^24, |x| < 2^67
-GL_HD W3 mul_2_24(const W3& x) {
+// x 2^S for S < 32, |x| < 2^(95 - S)
+template <int S>
+GL_HD W3 mul_low(const W3& x) {
+  static_assert(S > 0 && S < 32, "shift range");
 #if defined(__CUDA_ARCH__)
-  return {x.a0 << 24, __funnelshift_l(x.a0, x.a1, 24), __funnelshift_l(x.a1, x.a2, 24)};
+  return {x.a0 << S, __funnelshift_l(x.a0, x.a1, S), __funnelshift_l(x.a1, x.a2, S)};
 #else
-  return from_int(to_int(x) * ((__int128)1 << 24));
+  return from_int(to_int(x) * ((__int128)1 << S));
 #endif
 }
+GL_HD W3 mul_2_24(const W3& x) { return mul_low<24>(x); }
 
-// x 2^48, |x| < 2^79.  With (l2 : l1 : l0) = x 2^16 it is l0 2^32 + l1 2^64 + l2 2^96 =
-// l0 2^32 + l1 (2^32 - 1) - l2.
-GL_HD W3 mul_2_48(const W3& x) {
+// x 2^S for 32 < S < 64, |x| < 2^(127 - S); the result is below 2^65 + 2^33 in magnitude.  With
+// (l2 : l1 : l0) = x 2^(S - 32) it is l0 2^32 + l1 2^64 + l2 2^96 = l0 2^32 + l1 (2^32 - 1) - l2.
+template <int S>
+GL_HD W3 mul_mid(const W3& x) {
+  static_assert(S > 32 && S < 64, "shift range");
 #if defined(__CUDA_ARCH__)
-  const uint32_t l0 = x.a0 << 16, l1 = __funnelshift_l(x.a0, x.a1, 16), l2 = __funnelshift_l(x.a1, x.a2, 16);
+  const uint32_t l0 = x.a0 << (S - 32), l1 = __funnelshift_l(x.a0, x.a1, S - 32),
+                 l2 = __funnelshift_l(x.a1, x.a2, S - 32);
   const uint32_t sg = sign_word(x.a2);
   W3 r;
   asm("mad.lo.cc.u32  %0, %4, 0xFFFFFFFF, 0;\n\t"
@@ -120,17 +126,22 @@ GL_HD W3 mul_2_48(const W3& x) {
       : "r"(l0), "r"(l1), "r"(l2), "r"(sg));
   return r;
 #else
-  const __int128 l = to_int(x) * 65536;
+  const __int128 l = to_int(x) * ((__int128)1 << (S - 32));
+  from_int(l);
   const __int128 l0 = (uint32_t)l, l1 = (uint32_t)(l >> 32), l2 = l >> 64;
   return from_int((l0 << 32) + l1 * 0xFFFFFFFFll - l2);
 #endif
 }
+GL_HD W3 mul_2_48(const W3& x) { return mul_mid<48>(x); }
 
-// x 2^72, |x| < 2^87.  With (e2 : e1 : e0) = x 2^8 it is e0 2^64 + e1 2^96 + e2 2^128 =
-// (e0 - e2) 2^32 - e0 - e1.
-GL_HD W3 mul_2_72(const W3& x) {
+// x 2^S for 64 < S < 96, |x| < 2^(159 - S); the result is below 2^65 in magnitude.  With
+// (e2 : e1 : e0) = x 2^(S - 64) it is e0 2^64 + e1 2^96 + e2 2^128 = (e0 - e2) 2^32 - e0 - e1.
+template <int S>
+GL_HD W3 mul_high(const W3& x) {
+  static_assert(S > 64 && S < 96, "shift range");
 #if defined(__CUDA_ARCH__)
-  const uint32_t e0 = x.a0 << 8, e1 = __funnelshift_l(x.a0, x.a1, 8), e2 = __funnelshift_l(x.a1, x.a2, 8);
+  const uint32_t e0 = x.a0 << (S - 64), e1 = __funnelshift_l(x.a0, x.a1, S - 64),
+                 e2 = __funnelshift_l(x.a1, x.a2, S - 64);
   const uint32_t sg = sign_word(x.a2);
   W3 r;
   asm("sub.cc.u32  %0, 0, %3;\n\t"
@@ -143,11 +154,13 @@ GL_HD W3 mul_2_72(const W3& x) {
       : "r"(e0), "r"(e1), "r"(e2), "r"(sg));
   return r;
 #else
-  const __int128 e = to_int(x) * 256;
+  const __int128 e = to_int(x) * ((__int128)1 << (S - 64));
+  from_int(e);
   const __int128 e0 = (uint32_t)e, e1 = (uint32_t)(e >> 32), e2 = e >> 64;
   return from_int((e0 - e2) * ((__int128)1 << 32) - e0 - e1);
 #endif
 }
+GL_HD W3 mul_2_72(const W3& x) { return mul_high<72>(x); }
 
 // 0 <= x < 2^95 to a congruent 64-bit word: (a1 : a0) + a2 (2^32 - 1), whose carry c
 // comes back as c (2^32 - 1): with c = 1 the wrapped sum is below 2^63, so that cannot wrap.
@@ -304,28 +317,38 @@ GL_HD void dif(W3 (&x)[R], uint64_t (&out)[R]) {
       out[7] = reduce(sub(f, y));
     }
   } else {
-    // one stage with the twiddles 2^(12 k), its differences reduced to words, then two 8-point halves
-    W3 h[8];
-    uint64_t o[8];
+    // 4 x 4: 4-point transforms at stride 4, twiddles 2^(12 k1 n2), 4-point transforms.  A twiddle
+    // of 2^24 leaves 2^91, which 2^48 may not be applied to: the k1 = 2 column takes 2^72 and 2^24 of
+    // the untwiddled values instead, as the 8-point transform does.
+    W3 a[4][4];  // [k1][n2]
+    x[0] = add_bias(x[0]);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      h[k] = add(x[k], x[k + 8]);
-      x[k + 8] = sub(x[k], x[k + 8]);
+    for (int n2 = 0; n2 < 4; ++n2) {
+      const W3 s0 = add(x[n2], x[n2 + 8]), d0 = sub(x[n2], x[n2 + 8]), s1 = add(x[n2 + 4], x[n2 + 12]);
+      const W3 d1 = mul_2_48(sub(x[n2 + 4], x[n2 + 12]));
+      a[0][n2] = add(s0, s1);
+      a[2][n2] = sub(s0, s1);
+      a[1][n2] = add(d0, d1);
+      a[3][n2] = sub(d0, d1);
     }
-    dif<8>(h, o);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) out[k] = o[k];
-    h[0] = x[8];
-    h[1] = from_word(shl_c<12>(reduce(add_bias(x[9]))));
-    h[2] = from_word(shl_c<24>(reduce(add_bias(x[10]))));
-    h[3] = from_word(shl_c<36>(reduce(add_bias(x[11]))));
-    h[4] = from_word(shl_c<48>(reduce(add_bias(x[12]))));
-    h[5] = from_word(shl_c<60>(reduce(add_bias(x[13]))));
-    h[6] = from_word(shl_c<72>(reduce(add_bias(x[14]))));
-    h[7] = from_word(shl_c<84>(reduce(add_bias(x[15]))));
-    dif<8>(h, o);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) out[8 + k] = o[k];
+    auto last = [&](const W3& b0, const W3& b2, const W3& sum13, const W3& diff13, int o) {
+      const W3 s = add(b0, b2), d = sub(b0, b2);
+      out[o] = reduce(add(s, sum13));
+      out[o + 1] = reduce(sub(s, sum13));
+      out[o + 2] = reduce(add(d, diff13));
+      out[o + 3] = reduce(sub(d, diff13));
+    };
+    last(a[0][0], a[0][2], add(a[0][1], a[0][3]), mul_2_48(sub(a[0][1], a[0][3])), 0);
+    last(a[2][0], mul_2_48(a[2][2]), add(mul_2_24(a[2][1]), mul_2_72(a[2][3])),
+         add(mul_2_72(a[2][1]), mul_2_24(a[2][3])), 4);
+    {
+      const W3 b1 = mul_low<12>(a[1][1]), b3 = mul_mid<36>(a[1][3]);
+      last(a[1][0], mul_2_24(a[1][2]), add(b1, b3), mul_2_48(sub(b1, b3)), 8);
+    }
+    {
+      const W3 b1 = mul_mid<36>(a[3][1]), b3 = mul_low<12>(a[3][3]);  // 2^108 = -2^12
+      last(a[3][0], mul_2_72(a[3][2]), sub(b1, b3), mul_2_48(add(b1, b3)), 12);
+    }
   }
 }
 
@@ -370,24 +393,50 @@ GL_HD void dit_inv(W3 (&x)[R], uint64_t (&out)[R]) {
       out[7] = reduce(add(e, z));
     }
   } else {
-    W3 h[8];
-    uint64_t lo[8], hi[8];
+    // the steps of dif<16> backwards; inverse twiddles 2^-e = -2^(96 - e), 2^-108 = 2^84
+    W3 c[4][4];  // [k1][n2]
+    x[0] = add_bias(x[0]);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) h[k] = x[k];
-    dit_inv<8>(h, lo);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) h[k] = x[8 + k];
-    dit_inv<8>(h, hi);
-    // last stage: inverse twiddles 2^-12k = -2^(96 - 12 k)
-    const W3 t[8] = {from_word(shl_c<0>(hi[0])),  from_word(shl_c<84>(hi[1])), from_word(shl_c<72>(hi[2])),
-                     from_word(shl_c<60>(hi[3])), from_word(shl_c<48>(hi[4])), from_word(shl_c<36>(hi[5])),
-                     from_word(shl_c<24>(hi[6])), from_word(shl_c<12>(hi[7]))};
-    out[0] = reduce(add(from_word(lo[0]), t[0]));
-    out[8] = reduce(add_bias(sub(from_word(lo[0]), t[0])));
-#pragma unroll
-    for (int k = 1; k < 8; ++k) {
-      out[k] = fold(sub(from_word(lo[k]), t[k]));
-      out[k + 8] = fold(add(from_word(lo[k]), t[k]));
+    for (int o = 0; o < 4; ++o) {
+      const int k1 = (o >> 1) | ((o & 1) << 1);
+      const W3 p0 = add(x[4 * o], x[4 * o + 1]), p1 = sub(x[4 * o], x[4 * o + 1]);
+      const W3 p2 = add(x[4 * o + 2], x[4 * o + 3]), p3 = mul_2_48(sub(x[4 * o + 2], x[4 * o + 3]));
+      c[k1][0] = add(p0, p2);
+      c[k1][2] = sub(p0, p2);
+      c[k1][1] = sub(p1, p3);
+      c[k1][3] = add(p1, p3);
+    }
+    // s, d: terms 0 +- 2; sum13: terms 1 + 3; diff13: 2^48 (term 1 - term 3)
+    auto last = [&](const W3& s, const W3& d, const W3& sum13, const W3& diff13, int o) {
+      out[o] = reduce(add(s, sum13));
+      out[o + 8] = reduce(sub(s, sum13));
+      out[o + 4] = reduce(sub(d, diff13));
+      out[o + 12] = reduce(add(d, diff13));
+    };
+    // the same with sum13 and diff13 negated
+    auto last_neg = [&](const W3& s, const W3& d, const W3& sum13, const W3& diff13, int o) {
+      out[o] = reduce(sub(s, sum13));
+      out[o + 8] = reduce(add(s, sum13));
+      out[o + 4] = reduce(add(d, diff13));
+      out[o + 12] = reduce(sub(d, diff13));
+    };
+    last(add(c[0][0], c[2][0]), sub(c[0][0], c[2][0]), add(c[1][0], c[3][0]), mul_2_48(sub(c[1][0], c[3][0])), 0);
+    {
+      const W3 t2 = mul_2_72(c[2][1]), t1 = mul_high<84>(c[1][1]), t3 = mul_mid<60>(c[3][1]);
+      last_neg(sub(c[0][1], t2), add(c[0][1], t2), add(t1, t3), mul_2_48(sub(t1, t3)), 1);
+    }
+    {
+      // terms 1 + 3: -(2^72 c1 + 2^24 c3); 2^48 (term 1 - term 3): 2^24 c1 + 2^72 c3
+      const W3 t2 = mul_2_48(c[2][2]), s = sub(c[0][2], t2), d = add(c[0][2], t2);
+      const W3 f = add(mul_2_72(c[1][2]), mul_2_24(c[3][2])), g = add(mul_2_24(c[1][2]), mul_2_72(c[3][2]));
+      out[2] = reduce(sub(s, f));
+      out[10] = reduce(add(s, f));
+      out[6] = reduce(sub(d, g));
+      out[14] = reduce(add(d, g));
+    }
+    {
+      const W3 t2 = mul_2_24(c[2][3]), t1 = mul_mid<60>(c[1][3]), t3 = mul_high<84>(c[3][3]);
+      last_neg(sub(c[0][3], t2), add(c[0][3], t2), sub(t1, t3), mul_2_48(add(t1, t3)), 3);
     }
   }
 }

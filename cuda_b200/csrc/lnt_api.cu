@@ -48,6 +48,7 @@ struct lnt_test {
   uint64_t *twf = nullptr, *twi = nullptr;
   uint64_t *rt1 = nullptr, *irt1 = nullptr, *rt2 = nullptr, *irt2 = nullptr;
   uint64_t *itw1 = nullptr, *iitw1 = nullptr, *itw2 = nullptr, *iitw2 = nullptr;
+  uint64_t *itw1x = nullptr, *iitw1x = nullptr;  // rows that also run 16-point passes
   uint64_t *tw5 = nullptr, *itw5 = nullptr;  // n = 5 * 2^k: the radix-5 step's twiddles
   uint64_t c5[4] = {};                        // and its constants
   uint64_t* pw = nullptr;  // omega_n^e of the cluster kernel (512 ... 32768 words, policy plans)
@@ -122,7 +123,7 @@ void free_all(lnt_test* t) {
   free_jacobi(t);
   void* ptrs[] = {t->x, t->w, t->uw, t->widths, t->status, t->rt, t->irt, t->rdesc, t->tdesc,
                   t->twf, t->twi, t->rt1, t->irt1, t->rt2, t->irt2, t->itw1, t->iitw1,
-                  t->itw2, t->iitw2, t->tw5, t->itw5, t->rowf, t->colw, t->colf, t->pw, t->carry, t->fuse, t->canon,
+                  t->itw2, t->iitw2, t->itw1x, t->iitw1x, t->tw5, t->itw5, t->rowf, t->colw, t->colf, t->pw, t->carry, t->fuse, t->canon,
                   t->blk_carry, t->blk_fn, t->blk_cin, t->cflags};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -234,6 +235,8 @@ lnt::TwoPassDesc twopass_desc(const lnt_test* t) {
   d.five = t->plan.five ? 1 : 0;
   d.tw5 = t->tw5;
   d.itw5 = t->itw5;
+  d.itw1x = t->itw1x;
+  d.iitw1x = t->iitw1x;
   for (int k = 0; k < 4; ++k) d.c5[k] = t->c5[k];
   return d;
 }
@@ -1014,6 +1017,7 @@ uint64_t test_device_bytes(uint32_t n) {
     b += 16ull * n + 8ull * (plan.n1 + plan.n2) + 2ull * n + sizeof(TwoPassDesc) +
          4ull * (plan.n1 + 2);  // fused-kernel flags
     if (plan.fast) b += 36ull * plan.n1 + 48ull * plan.n2;  // inner twiddles, weight factors
+    if (plan.fast && r16_row_radix(plan.radix, plan.n1) == 16) b += 24ull * plan.n1;  // 16-point row passes
     if (plan.five) b += 64ull * (plan.n1 / 5);                      // radix-5 twiddles
   }
   return b;
@@ -1132,12 +1136,16 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
     if (plan.fast) {
       // pass tables of the row transform: n1 points, or L = n1 / 5 for each plane of a 5 * 2^k row
       const uint32_t row_points = plan.five ? plan.n1 / 5 : plan.n1;
-      if ((st = upload_roots(t, row_points, &t->itw1, &t->iitw1, plan.radix)) != LNT_OK) return bail(st);
+      if ((st = upload_roots(t, row_points, &t->itw1, &t->iitw1, 8)) != LNT_OK) return bail(st);
+      if (lnt::r16_row_radix(plan.radix, plan.n1) == 16 &&
+          (st = upload_roots(t, plan.n1, &t->itw1x, &t->iitw1x, 16)) != LNT_OK)
+        return bail(st);
       if (plan.five &&
           ((e = dalloc(&t->tw5, 4 * (size_t)row_points)) || (e = dalloc(&t->itw5, 4 * (size_t)row_points)) ||
            (e = lnt::launch_five_twiddles(row_points, t->tw5, t->itw5, t->c5, t->stream))))
         return bail(cuda_fail(e, "radix-5 twiddles"));
-      if ((st = upload_roots(t, plan.n2, &t->itw2, &t->iitw2, plan.radix)) != LNT_OK) return bail(st);
+      if ((st = upload_roots(t, plan.n2, &t->itw2, &t->iitw2,
+                             lnt::r16_col_radix(plan.radix, plan.five, plan.n2))) != LNT_OK) return bail(st);
       if ((e = dalloc(&t->rowf, 2 * (size_t)plan.n2)) || (e = dalloc(&t->colf, plan.n1)) ||
           (e = dalloc(&t->colw, plan.n1)) ||
           (e = lnt::launch_weight_factors(exponent, plan.n1, plan.n2, t->rowf, t->colf, t->colw, t->stream)))

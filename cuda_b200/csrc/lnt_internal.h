@@ -177,13 +177,16 @@ struct TwoPassDesc {
   uint32_t* fuse;
   uint32_t n1, n2, log2n1, log2n2, tile, ntiles;
   uint32_t prp;
-  uint32_t radix;  // largest pass radix of the row and column transforms: 8 or 16
+  uint32_t radix;  // the plan's pass radix, 8 or 16 (r16_row_radix, r16_col_radix)
   // n = 5 * 2^k (five != 0): n1 = 5 L and log2n1 = log2 L.  tw5[(k5 - 1) L + c] =
   // omega_{5L}^(k5 c) for plane k5 = 1..4 and plane position c, itw5 its
   // inverse; c5 = the constants of lazy::dft5 (lazy_core.cuh)
   uint32_t five;
   const uint64_t* tw5;
   const uint64_t* itw5;
+  // rows that also run passes of 16 points (r16_row_radix): those passes' twiddles
+  const uint64_t* itw1x;
+  const uint64_t* iitw1x;
   uint64_t c5[4];
 };
 
@@ -197,6 +200,10 @@ bool r16_supported(uint32_t log2n1, uint32_t log2n2);
 // radices of the passes of a length-2^log2L transform whose passes take at most
 // `radix` (8 or 16) points, first (largest span) first
 std::vector<uint32_t> r16_pass_radices(uint32_t log2L, uint32_t radix);
+// The largest pass radix that the columns (n2 words) of a plan take, and that its rows (n1 words) take
+// in launches of few CTAs (8 in larger ones); lnt_radix16.cu says where the lines lie.
+uint32_t r16_row_radix(uint32_t plan_radix, uint32_t n1);
+uint32_t r16_col_radix(uint32_t plan_radix, bool five, uint32_t n2);
 uint32_t r16_tile(uint32_t log2n2);
 uint32_t r16_run_words_needed(uint32_t exponent, uint32_t n);
 // `d` gives the geometry (shared by every test of the launch); `dd` is a device

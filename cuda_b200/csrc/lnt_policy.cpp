@@ -239,7 +239,9 @@ bool make_plan(uint32_t n, uint32_t exponent, const PlanOptions* opt, Plan& plan
   plan.tile = tile;
   plan.ntiles = plan.n1 / plan.tile;
   if (plan.fast) {
-    plan.radix = o.radix ? o.radix : 8;
+    // policy: passes of up to 16 points from 2^19 words on, where columns or rows of 1024 and more
+    // words save a pass (r16_row_radix, r16_col_radix)
+    plan.radix = o.radix ? o.radix : (plan.log2n >= 19 ? 16 : 8);
     // policy: the carry-fused column kernel from 2^19 words, where its tiles
     // fill the GPU; the autotuner may choose either way at any length
     plan.fused = o.fused ? o.fused == 1 : plan.log2n >= 19;

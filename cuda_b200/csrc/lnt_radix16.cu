@@ -39,16 +39,14 @@ constexpr int row_square_threads(int L, int rows, bool latency) {
                   : (L * rows >= 4096 || latency ? 256
                                                  : (L * rows >= 2048 ? 128 : (L * rows >= 1024 ? 64 : 32)));
 }
-#ifndef LNT_ROW_MIN_BLOCKS
-#define LNT_ROW_MIN_BLOCKS 4  // CTAs per SM the row kernel is compiled for (registers)
-#endif
-// Radix-16 passes hold 16 values and their twiddles per thread: at the 64
-// registers of four row CTAs (two 4-column CTAs) per SM they spill, so their
-// kernels are built for half the CTAs per SM (128 registers, no spills).
-template <int TH, int MR>
-constexpr int row_min_blocks() {
-  return TH == 256 ? (MR == 16 ? 2 : LNT_ROW_MIN_BLOCKS)
-                   : ((MR == 16 ? 512 : 1024) / TH > 0 ? (MR == 16 ? 512 : 1024) / TH : 1);
+// CTAs of TH threads an SM that the kernels are compiled for.  Passes of up to 8 points: 1024 threads,
+// 64 registers.  Passes of 16 points hold 48 registers of three-word values and the twiddles: 512
+// threads, 128 registers.  `Dense`: 768 threads, 80 registers; they spill (264 bytes in col_fused), which
+// only a launch of many CTAs makes up for (col_dense).
+template <int TH, int MR, bool Dense = false>
+constexpr int min_blocks() {
+  constexpr int threads = MR == 16 ? (Dense ? 768 : 512) : 1024;
+  return threads / TH > 0 ? threads / TH : 1;
 }
 
 // Forward pass of `rows` row transforms.  The first pass (span = L) reads HBM
@@ -161,8 +159,14 @@ __device__ __forceinline__ void row_pass_r(int R, uint64_t* sm, int ld, int rows
   }
 }
 
+// the pass tables of a row of n1 words
+template <int MR>
+__device__ __forceinline__ const uint64_t* row_tw(const TwoPassDesc& D) { return MR == 16 ? D.itw1x : D.itw1; }
+template <int MR>
+__device__ __forceinline__ const uint64_t* row_itw(const TwoPassDesc& D) { return MR == 16 ? D.iitw1x : D.iitw1; }
+
 template <int TH, int MR>
-__global__ void __launch_bounds__(TH, row_min_blocks<TH, MR>()) row_square_r16(const TwoPassDesc* __restrict__ Ds, Passes P, int rows) {
+__global__ void __launch_bounds__(TH, min_blocks<TH, MR>()) row_square_r16(const TwoPassDesc* __restrict__ Ds, Passes P, int rows) {
   extern __shared__ __align__(16) uint64_t sm[];
   const TwoPassDesc& D = Ds[blockIdx.y];
   const int L = (int)D.n1, ld = padded(L);
@@ -170,7 +174,7 @@ __global__ void __launch_bounds__(TH, row_min_blocks<TH, MR>()) row_square_r16(c
   uint64_t* x = reinterpret_cast<uint64_t*>(D.x) + off;
   int span = L;
   for (int j = 0, seg = 0; j + 1 < P.m; ++j) {
-    row_pass_r<true, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twf + off, D.itw1 + seg);
+    row_pass_r<true, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twf + off, row_tw<MR>(D) + seg);
     seg += span;
     span /= P.radix[j];
     __syncthreads();
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(TH, row_min_blocks<TH, MR>()) row_square_r16(c
   for (int j = P.m - 2; j >= 0; --j) {
     span *= P.radix[j];
     row_pass_r<false, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twi + off,
-                      D.iitw1 + pass_table_offset(P, L, j));
+                      row_itw<MR>(D) + pass_table_offset(P, L, j));
     if (j) __syncthreads();
   }
 }
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(TH) row_forward_r16(const TwoPassDesc* __restr
   uint64_t* x = reinterpret_cast<uint64_t*>(D.x) + off;
   int span = L;
   for (int j = 0, seg = 0; j < P.m; ++j) {
-    row_pass_r<true, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twf + off, D.itw1 + seg);
+    row_pass_r<true, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twf + off, row_tw<MR>(D) + seg);
     seg += span;
     span /= P.radix[j];
     __syncthreads();
@@ -221,7 +225,7 @@ __global__ void __launch_bounds__(TH) row_mul_r16(const TwoPassDesc* __restrict_
   uint64_t* x = reinterpret_cast<uint64_t*>(D.x) + off;
   int span = L;
   for (int j = 0, seg = 0; j + 1 < P.m; ++j) {
-    row_pass_r<true, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twf + off, D.itw1 + seg);
+    row_pass_r<true, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twf + off, row_tw<MR>(D) + seg);
     seg += span;
     span /= P.radix[j];
     __syncthreads();
@@ -231,7 +235,7 @@ __global__ void __launch_bounds__(TH) row_mul_r16(const TwoPassDesc* __restrict_
   for (int j = P.m - 2; j >= 0; --j) {
     span *= P.radix[j];
     row_pass_r<false, MR>(P.radix[j], sm, ld, rows, L, span, x, D.twi + off,
-                      D.iitw1 + pass_table_offset(P, L, j));
+                      row_itw<MR>(D) + pass_table_offset(P, L, j));
     if (j) __syncthreads();
   }
 }
@@ -333,17 +337,15 @@ __global__ void __launch_bounds__(TH) row5_r16(const TwoPassDesc* __restrict__ D
 // instead of CTAs whose threads mostly idle.  A launch with fewer CTAs than
 // twice the SMs (one short test: latency) keeps 128 threads a column, whose
 // row-wise steps (carries, weights, staging) then run in parallel.
+// 16-point passes (columns of 1024 and more words) take half the threads at twice the registers.
+template <int MR>
 __host__ __device__ constexpr int col_tpc(uint32_t n2, bool latency) {
+  if (MR == 16) return n2 >= 4096 ? 128 : 64;
   return n2 >= 4096 ? 256 : (n2 >= 1024 || latency ? 128 : (n2 == 512 ? 64 : 32));
 }
 inline bool col_latency_mode(const TwoPassDesc& d, uint32_t count) {
   return (uint64_t)d.ntiles * count < 2ull * device_sms();
 }
-// CTAs per SM the column kernels are compiled for: 64 registers a thread at
-// 1024 threads an SM (128 for radix-16 passes, which spill at 64)
-template <int TH, int MR>
-constexpr int col_min_blocks() { return (MR == 16 ? 512 : 1024) / TH > 0 ? (MR == 16 ? 512 : 1024) / TH : 1; }
-
 // words of shared memory of a tile of T columns of L words (smem::Tile)
 __host__ __device__ constexpr size_t tile_words(int L, int T) { return (size_t)T * (L + L / 8); }
 
@@ -533,7 +535,7 @@ __device__ __forceinline__ void inverse_tile(const TwoPassDesc& D, const Passes&
 }
 
 template <int T, int TH, int MR>
-__global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_forward_r16(
+__global__ void __launch_bounds__(TH, min_blocks<TH, MR>()) col_forward_r16(
     const TwoPassDesc* __restrict__ Ds, Passes P, int apply_carries) {
   extern __shared__ __align__(16) uint64_t sm[];
   const TwoPassDesc& D = Ds[blockIdx.y];
@@ -546,7 +548,7 @@ __global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_forward_r16(
 }
 
 template <int T, int TH, int MR>
-__global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_inverse_r16(
+__global__ void __launch_bounds__(TH, min_blocks<TH, MR>()) col_inverse_r16(
     const TwoPassDesc* __restrict__ Ds, Passes P, int unsigned_mode) {
   extern __shared__ __align__(16) uint64_t sm[];
   const TwoPassDesc& D = Ds[blockIdx.y];
@@ -616,8 +618,8 @@ __device__ __forceinline__ void wait_flag(const uint32_t* flag, uint32_t want, u
   __syncthreads();
 }
 
-template <int T, int TH, int MR>
-__global__ void __launch_bounds__(TH, col_min_blocks<TH, MR>()) col_fused_r16(
+template <int T, int TH, int MR, bool Dense>
+__global__ void __launch_bounds__(TH, min_blocks<TH, MR, Dense>()) col_fused_r16(
     const TwoPassDesc* __restrict__ Ds, Passes P) {
   extern __shared__ __align__(16) uint64_t sm[];
   __shared__ uint32_t s_ticket, s_epoch;
@@ -737,8 +739,27 @@ uint32_t r16_run_words_needed(uint32_t exponent, uint32_t n) {
   return (log2n + wmax + wmin - 2) / (wmin - 1) + 1;
 }
 
-// log2 of the largest pass radix of a descriptor's plan (3: radix 8, 4: radix 16)
-inline int radix_log2(const TwoPassDesc& d) { return d.radix == 16 ? 4 : 3; }
+// Passes of 16 points save one pass (and a quarter of the general products) of a transform of 1024,
+// 2048 or 4096 words, at twice the registers.  Columns gain from it (col_fused, us, 8 -> 16 points:
+// n2 = 1024 40.8 -> 36.9 at n = 2^20, 2048 188.8 -> 178 at 2^23, 4096 408 -> 389 at 2^24 and 1603 ->
+// 1509 at 2^26; 512 words save no pass: 24.5 -> 28.5 at 2^19).  Lengths 5 * 2^k have no radix option;
+// their columns follow the same line.
+uint32_t r16_col_radix(uint32_t plan_radix, bool five, uint32_t n2) {
+  return (plan_radix == 16 || five) && n2 >= 1024 ? 16 : 8;
+}
+// Rows of 1024 and 2048 words gain only in a launch that leaves registers idle, below four CTAs an SM
+// (row_square, us: 32.7 -> 26.5 at 2^20, 51.1 -> 47.0 at 2^21; 1024 CTAs of 2048 words, 2^22, 88 -> 104);
+// such plans keep the pass tables of both radices.  Rows of 4096 words and more lose (157.9 -> 182.1 at
+// 2^23): their first and last passes, whose 16 words and 16 twiddles a task come from HBM, find too few
+// warps to hide it.
+uint32_t r16_row_radix(uint32_t plan_radix, uint32_t n1) {
+  return plan_radix == 16 && (n1 == 1024 || n1 == 2048) ? 16 : 8;
+}
+bool rows16(const TwoPassDesc& d, uint32_t count) {
+  return r16_row_radix(d.radix, d.n1) == 16 &&
+         (uint64_t)(d.n2 / row_rows_per_cta((int)d.n1, (int)d.n2, count)) * count < 4ull * device_sms();
+}
+bool cols16(const TwoPassDesc& d) { return r16_col_radix(d.radix, d.five != 0, d.n2) == 16; }
 
 template <int TH, int MR>
 cudaError_t row_square_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count, cudaStream_t s) {
@@ -746,7 +767,7 @@ cudaError_t row_square_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t c
   const size_t smem = (size_t)rows * padded(L) * 8;
   cudaError_t e = ensure_smem(row_square_r16<TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  row_square_r16<TH, MR><<<dim3(d.n2 / rows, count), TH, smem, s>>>(dd, make_passes((int)d.log2n1, radix_log2(d)), rows);
+  row_square_r16<TH, MR><<<dim3(d.n2 / rows, count), TH, smem, s>>>(dd, make_passes((int)d.log2n1, MR == 16 ? 4 : 3), rows);
   return cudaGetLastError();
 }
 
@@ -756,7 +777,7 @@ cudaError_t row_forward_t(const TwoPassDesc& d, const TwoPassDesc* dd, cudaStrea
   const size_t smem = (size_t)rows * padded(L) * 8;
   cudaError_t e = ensure_smem(row_forward_r16<TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  row_forward_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(dd, make_passes((int)d.log2n1, radix_log2(d)), rows);
+  row_forward_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(dd, make_passes((int)d.log2n1, MR == 16 ? 4 : 3), rows);
   return cudaGetLastError();
 }
 
@@ -766,13 +787,15 @@ cudaError_t row_mul_t(const TwoPassDesc& d, const TwoPassDesc* dd, const uint64_
   const size_t smem = (size_t)rows * padded(L) * 8;
   cudaError_t e = ensure_smem(row_mul_r16<TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  row_mul_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(dd, make_passes((int)d.log2n1, radix_log2(d)), rows, F);
+  row_mul_r16<TH, MR><<<dim3(d.n2 / rows, 1), TH, smem, s>>>(dd, make_passes((int)d.log2n1, MR == 16 ? 4 : 3), rows, F);
   return cudaGetLastError();
 }
 
+// 16-point passes: rows of 1024 or 2048 words only (r16_row_radix), 256 threads and fewer
 template <int MR>
 cudaError_t row_forward_m(const TwoPassDesc& d, const TwoPassDesc* dd, cudaStream_t s) {
-  switch (row_threads_for((int)d.n1)) {
+  if constexpr (MR == 16) return row_forward_t<256, MR>(d, dd, s);
+  else switch (row_threads_for((int)d.n1)) {
     case 256: return row_forward_t<256, MR>(d, dd, s);
     case 512: return row_forward_t<512, MR>(d, dd, s);
     default: return row_forward_t<1024, MR>(d, dd, s);
@@ -781,7 +804,8 @@ cudaError_t row_forward_m(const TwoPassDesc& d, const TwoPassDesc* dd, cudaStrea
 
 template <int MR>
 cudaError_t row_mul_m(const TwoPassDesc& d, const TwoPassDesc* dd, const uint64_t* F, cudaStream_t s) {
-  switch (row_threads_for((int)d.n1)) {
+  if constexpr (MR == 16) return row_mul_t<256, MR>(d, dd, F, s);
+  else switch (row_threads_for((int)d.n1)) {
     case 256: return row_mul_t<256, MR>(d, dd, F, s);
     case 512: return row_mul_t<512, MR>(d, dd, F, s);
     default: return row_mul_t<1024, MR>(d, dd, F, s);
@@ -793,13 +817,19 @@ cudaError_t row_square_m(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t c
   const int rows = row_rows_per_cta((int)d.n1, (int)d.n2, count);
   const bool latency = (uint64_t)(d.n2 / rows) * count < 2ull * device_sms();
   switch (row_square_threads((int)d.n1, rows, latency)) {
-    case 32: return row_square_t<32, MR>(d, dd, count, s);
     case 64: return row_square_t<64, MR>(d, dd, count, s);
     case 128: return row_square_t<128, MR>(d, dd, count, s);
     case 256: return row_square_t<256, MR>(d, dd, count, s);
-    case 512: return row_square_t<512, MR>(d, dd, count, s);
-    default: return row_square_t<1024, MR>(d, dd, count, s);
+    default: break;
   }
+  if constexpr (MR == 8) {
+    switch (row_square_threads((int)d.n1, rows, latency)) {
+      case 32: return row_square_t<32, MR>(d, dd, count, s);
+      case 512: return row_square_t<512, MR>(d, dd, count, s);
+      default: return row_square_t<1024, MR>(d, dd, count, s);
+    }
+  }
+  return cudaErrorInvalidConfiguration;
 }
 
 // Rows of 5 L words (radix-8 passes) per CTA: as many as fit 4096 words (a
@@ -832,31 +862,35 @@ cudaError_t row5_launch(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t co
 
 cudaError_t launch_row_forward_r16(const TwoPassDesc& d, const TwoPassDesc* dd, cudaStream_t s) {
   if (d.five) return row5_launch<1>(d, dd, 1, nullptr, s);
-  return d.radix == 16 ? row_forward_m<16>(d, dd, s) : row_forward_m<8>(d, dd, s);
+  return rows16(d, 1) ? row_forward_m<16>(d, dd, s) : row_forward_m<8>(d, dd, s);
 }
 
 cudaError_t launch_row_mul_r16(const TwoPassDesc& d, const TwoPassDesc* dd, const uint64_t* F,
                                cudaStream_t s) {
   if (d.five) return row5_launch<2>(d, dd, 1, F, s);
-  return d.radix == 16 ? row_mul_m<16>(d, dd, F, s) : row_mul_m<8>(d, dd, F, s);
+  return rows16(d, 1) ? row_mul_m<16>(d, dd, F, s) : row_mul_m<8>(d, dd, F, s);
 }
 
 cudaError_t launch_row_square_r16(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count,
                                   cudaStream_t s) {
   if (d.five) return row5_launch<0>(d, dd, count, nullptr, s);
-  return d.radix == 16 ? row_square_m<16>(d, dd, count, s) : row_square_m<8>(d, dd, count, s);
+  return rows16(d, count) ? row_square_m<16>(d, dd, count, s) : row_square_m<8>(d, dd, count, s);
 }
 
 // The column kernels' thread count for a tile of T columns of n2 words.
-template <int T, class F>
+template <int T, int MR, class F>
 cudaError_t col_dispatch(uint32_t n2, bool latency, F&& f) {
-  switch (T * col_tpc(n2, latency)) {
+  switch (T * col_tpc<MR>(n2, latency)) {
     case 128:
-      if constexpr (T == 4) return f(std::integral_constant<int, 128>{});
+      if constexpr (T == 4 && MR == 8) return f(std::integral_constant<int, 128>{});
       break;
-    case 256: return f(std::integral_constant<int, 256>{});
+    case 256:
+      if constexpr (T == 4 || MR == 8) return f(std::integral_constant<int, 256>{});
+      break;
     case 512: return f(std::integral_constant<int, 512>{});
-    case 1024: return f(std::integral_constant<int, 1024>{});
+    case 1024:
+      if constexpr (MR == 8) return f(std::integral_constant<int, 1024>{});
+      break;
     default: break;
   }
   return cudaErrorInvalidConfiguration;
@@ -867,7 +901,7 @@ cudaError_t col_forward_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t 
   const size_t smem = tile_words((int)d.n2, T) * 8;
   cudaError_t e = ensure_smem(col_forward_r16<T, TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  col_forward_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, radix_log2(d)), apply ? 1 : 0);
+  col_forward_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, MR == 16 ? 4 : 3), apply ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -877,17 +911,25 @@ cudaError_t col_inverse_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t 
   const size_t smem = tile_words((int)d.n2, T) * 8;
   cudaError_t e = ensure_smem(col_inverse_r16<T, TH, MR>, smem);
   if (e != cudaSuccess) return e;
-  col_inverse_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, radix_log2(d)), unsigned_mode ? 1 : 0);
+  col_inverse_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, MR == 16 ? 4 : 3), unsigned_mode ? 1 : 0);
   return cudaGetLastError();
 }
 
-template <int T, int TH, int MR>
+template <int T, int TH, int MR, bool Dense>
 cudaError_t col_fused_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count, cudaStream_t s) {
   const size_t smem = tile_words((int)d.n2, T) * 8;
-  cudaError_t e = ensure_smem(col_fused_r16<T, TH, MR>, smem);
+  cudaError_t e = ensure_smem(col_fused_r16<T, TH, MR, Dense>, smem);
   if (e != cudaSuccess) return e;
-  col_fused_r16<T, TH, MR><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, radix_log2(d)));
+  col_fused_r16<T, TH, MR, Dense><<<dim3(d.ntiles, count), TH, smem, s>>>(dd, make_passes((int)d.log2n2, MR == 16 ? 4 : 3));
   return cudaGetLastError();
+}
+
+// 16-point passes of 4-word tiles up to 2048 rows (73 KB: three fit an SM): three CTAs an SM instead
+// of two where the launch has eight tiles an SM and more.  col_fused, two -> three, us: 2560 tiles of 1024
+// rows (n = 5 * 2^21) 246.7 -> 223.2, 1024 of 2048 (2^23) 180.4 -> 177.9; 512 of 2048 (2^22) 108.0 -> 113.3,
+// 512 of 1024 (2^21) 59.2 -> 65.8, where the third CTA saves no wave.
+bool col_dense(const TwoPassDesc& d, uint32_t count) {
+  return d.tile == 4 && d.n2 <= 2048 && (uint64_t)d.ntiles * count >= 8ull * device_sms();
 }
 
 // Tests per launch (the grid's y extent).  A CTA of the fused kernel waits only
@@ -897,8 +939,12 @@ constexpr uint32_t kFusedTestsPerLaunch = 1024;
 
 template <int T, int MR>
 cudaError_t col_fused_tm(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count, cudaStream_t s) {
-  return col_dispatch<T>(d.n2, col_latency_mode(d, count),
-                         [&](auto th) { return col_fused_t<T, decltype(th)::value, MR>(d, dd, count, s); });
+  return col_dispatch<T, MR>(d.n2, col_latency_mode(d, count), [&](auto th) {
+    constexpr int TH = decltype(th)::value;
+    if constexpr (MR == 16 && T == 4 && TH == 256)
+      if (col_dense(d, count)) return col_fused_t<T, TH, MR, true>(d, dd, count, s);
+    return col_fused_t<T, TH, MR, false>(d, dd, count, s);
+  });
 }
 
 template <int MR>
@@ -917,9 +963,9 @@ cudaError_t col_forward_m(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t 
                           cudaStream_t s) {
   const bool latency = col_latency_mode(d, count);
   if (d.tile == 8)
-    return col_dispatch<8>(d.n2, latency,
+    return col_dispatch<8, MR>(d.n2, latency,
                            [&](auto th) { return col_forward_t<8, decltype(th)::value, MR>(d, dd, count, apply, s); });
-  return col_dispatch<4>(d.n2, latency,
+  return col_dispatch<4, MR>(d.n2, latency,
                          [&](auto th) { return col_forward_t<4, decltype(th)::value, MR>(d, dd, count, apply, s); });
 }
 
@@ -928,28 +974,28 @@ cudaError_t col_inverse_m(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t 
                           bool unsigned_mode, cudaStream_t s) {
   const bool latency = col_latency_mode(d, count);
   if (d.tile == 8)
-    return col_dispatch<8>(d.n2, latency, [&](auto th) {
+    return col_dispatch<8, MR>(d.n2, latency, [&](auto th) {
       return col_inverse_t<8, decltype(th)::value, MR>(d, dd, count, unsigned_mode, s);
     });
-  return col_dispatch<4>(d.n2, latency, [&](auto th) {
+  return col_dispatch<4, MR>(d.n2, latency, [&](auto th) {
     return col_inverse_t<4, decltype(th)::value, MR>(d, dd, count, unsigned_mode, s);
   });
 }
 
 cudaError_t launch_col_fused_r16(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count,
                                  cudaStream_t s) {
-  return d.radix == 16 ? col_fused_m<16>(d, dd, count, s) : col_fused_m<8>(d, dd, count, s);
+  return cols16(d) ? col_fused_m<16>(d, dd, count, s) : col_fused_m<8>(d, dd, count, s);
 }
 
 cudaError_t launch_col_forward_r16(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count,
                                    bool apply, cudaStream_t s) {
-  return d.radix == 16 ? col_forward_m<16>(d, dd, count, apply, s)
+  return cols16(d) ? col_forward_m<16>(d, dd, count, apply, s)
                        : col_forward_m<8>(d, dd, count, apply, s);
 }
 
 cudaError_t launch_col_inverse_r16(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t count,
                                    bool unsigned_mode, cudaStream_t s) {
-  return d.radix == 16 ? col_inverse_m<16>(d, dd, count, unsigned_mode, s)
+  return cols16(d) ? col_inverse_m<16>(d, dd, count, unsigned_mode, s)
                        : col_inverse_m<8>(d, dd, count, unsigned_mode, s);
 }
 

@@ -50,11 +50,10 @@ struct Passes {
   int radix[6];   // r_0 (largest stride) ... r_{m-1} (contiguous)
 };
 
-// Default largest pass radix.  8 (three radix-2 stages per pass) keeps a task's
-// values, twiddles and addresses within the 64 registers that four row CTAs
-// (two column CTAs) per SM allow; 16 needs one twiddle stage less per direction
-// but spills there.  The two-pass kernels are built for both (a plan's `radix`)
-// and the autotuner picks per length; the resident kernel uses 8.
+// Default largest pass radix.  8 (three radix-2 stages per pass) keeps a task's values, twiddles and
+// addresses within the 64 registers that four row CTAs (two column CTAs) per SM allow; 16 needs one
+// twiddle stage less per direction and twice the registers.  The two-pass kernels are built for both
+// (r16_row_radix and r16_col_radix say which lengths take which); the resident kernel uses 8.
 constexpr int kDefaultRadixLog2 = 3;
 constexpr int kMaxRadix = 1 << kDefaultRadixLog2;
 

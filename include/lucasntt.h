@@ -103,7 +103,8 @@ typedef struct lnt_plan_options {
   uint32_t kind;      /* lnt_plan_kind */
   uint32_t log2_rows; /* two-pass: log2 of the column length n2 (n = n2 x n1); 0 = policy */
   uint32_t tile;      /* two-pass: columns per column CTA = words per carry run, 4 or 8; 0 = policy */
-  uint32_t radix;     /* LNT_PLAN_RADIX16: largest pass radix, 8 or 16; 0 = policy (8) */
+  uint32_t radix;     /* LNT_PLAN_RADIX16: largest pass radix, 8 or 16; 0 = policy
+                         (16 from 2^19 words) */
   uint32_t fused;     /* LNT_PLAN_RADIX16: 1 = the inverse column pass of a squaring and the
                          forward one of the next in one carry-fused launch, 2 = two launches;
                          0 = policy (fused from 2^19 words) */
@@ -123,7 +124,7 @@ int lnt_get_plan(lnt_test* t, lnt_plan_options* out);
  * plan for (q, n) (n = 0: policy length).  Writes min(count, cap) entries. */
 int lnt_plan_candidates(uint32_t exponent, uint32_t n, lnt_plan_options* out, int cap, int* count);
 
-/* Name of a plan ("TWOPASS_2048x4096_R8_T4": n2 x n1, pass radix, tile), the
+/* Name of a plan ("TWOPASS_2048x4096_R16_T4": n2 x n1, pass radix, tile), the
  * stats file's Pool line. */
 int lnt_plan_describe(const lnt_plan_options* plan, uint32_t exponent, uint32_t n, char* out,
                       size_t outlen);

@@ -92,3 +92,16 @@ def test_autotune_picks_a_working_plan(lnt):
         A.iterate(200)
         Bt.iterate(200)
         assert A.res64() == Bt.res64()
+
+
+@pytest.mark.parametrize("tile", [4, 8])
+@pytest.mark.parametrize("radix", [8, 16])
+def test_columns_of_2048_words(lnt, oracle_mod, radix, tile):
+    """The widest tiles: columns of 2048 words beside rows of 2048 (both lengths that take 16-point
+    passes), one launch a squaring for the columns and two."""
+    q, n = 75000017, 1 << 22
+    start = random_digits(q, n, 7)
+    want = oracle_digits(oracle_mod, q, n, True, start, 2)
+    for fused in (1, 2):
+        got, name = run_plan(lnt, q, n, True, (2, 11, tile, radix, fused), start, 2)
+        assert np.array_equal(got, want), name
