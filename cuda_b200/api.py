@@ -122,6 +122,7 @@ def lib() -> ctypes.CDLL:
         "lnt_gerbicz_stats": ([vp, ctypes.POINTER(u64), ctypes.POINTER(u64), ctypes.POINTER(u64)], i32),
         "lnt_debug_corrupt": ([vp, u32], i32),
         "lnt_debug_corrupt_add": ([vp, u32, ctypes.c_int64], i32),
+        "lnt_debug_cluster_quit": ([vp, u64, u64], i32),
         "lnt_batch_use_graphs": ([vp, i32], i32),
         "lnt_batch_short_lengths": ([vp, i32], i32),
         "lnt_batch_checkpoint_every": ([vp, u64], i32),
@@ -322,6 +323,11 @@ class LucasTest:
         """Test hook: add `delta` to one word of the device state (a simulated
         hardware error; a large delta makes the kernels raise the carry flag)."""
         _check(lib().lnt_debug_corrupt_add(self._h, int(word), int(delta)), "lnt_debug_corrupt_add")
+
+    def debug_cluster_quit(self, squaring: int, wait_ns: int = 50_000_000) -> None:
+        """Test hook: one CTA of the cluster kernel leaves before squaring `squaring` of a launch
+        (lnt_debug_cluster_quit)."""
+        _check(lib().lnt_debug_cluster_quit(self._h, int(squaring), int(wait_ns)), "lnt_debug_cluster_quit")
 
     def set_stream(self, stream_handle: int | None) -> None:
         _check(lib().lnt_set_stream(self._h, stream_handle), "lnt_set_stream")

@@ -51,6 +51,7 @@ struct lnt_test {
   uint64_t *itw1x = nullptr, *iitw1x = nullptr;  // rows that also run 16-point passes
   uint64_t *tw5 = nullptr, *itw5 = nullptr;  // n = 5 * 2^k: the radix-5 step's twiddles
   uint64_t c5[4] = {};                        // and its constants
+  uint64_t cluster_wait_ns = lnt::kClusterWaitNs, cluster_quit_at = ~0ull;  // lnt_debug_cluster_quit
   uint64_t* pw = nullptr;  // omega_n^e of the cluster kernel (512 ... 32768 words, policy plans)
   // separable weights of the register-pass column kernels (TwoPassDesc)
   ulonglong2 *rowf = nullptr, *colw = nullptr;
@@ -293,6 +294,8 @@ int check_status(lnt_test* t) {
     return fail(LNT_ERR_NUMERIC, "carry exceeded the balanced-digit headroom");
   if (t->h_pinned[0] & lnt::kStatusFuseTimeout)
     return fail(LNT_ERR_CUDA, "a carry-fused column CTA timed out waiting for its neighbour");
+  if (t->h_pinned[0] & lnt::kStatusClusterTimeout)
+    return fail(LNT_ERR_CUDA, "a CTA of the cluster kernel timed out waiting for words of another");
   return LNT_OK;
 }
 
@@ -461,6 +464,8 @@ lnt::ClusterDesc cluster_desc(const lnt_test* t, uint64_t iterations) {
     d.ntiles = t->plan.ntiles;
     if (t->pending_carries) d.carry = t->carry;
   }
+  d.wait_ns = t->cluster_wait_ns;
+  d.quit_at = t->cluster_quit_at;
   return d;
 }
 
@@ -1316,6 +1321,15 @@ int lnt_debug_corrupt_add(lnt_test* t, uint32_t word, int64_t delta) {
   LNT_CUDA(cudaMemcpyAsync(t->x + word, &v, 8, cudaMemcpyHostToDevice, t->stream), "write word");
   LNT_CUDA(cudaStreamSynchronize(t->stream), "synchronize");
   t->canon_valid = false;
+  return LNT_OK;
+}
+
+int lnt_debug_cluster_quit(lnt_test* t, uint64_t squaring, uint64_t wait_ns) {
+  if (!t || wait_ns == 0 || wait_ns > lnt::kClusterWaitNs)
+    return fail(LNT_ERR_INVALID_ARGUMENT, "null test, or a wait outside (0, 2 s]");
+  if (!cluster_plan(t->plan)) return fail(LNT_ERR_UNSUPPORTED_LENGTH, "the test does not run on the cluster kernel");
+  t->cluster_quit_at = squaring;
+  t->cluster_wait_ns = wait_ns;
   return LNT_OK;
 }
 

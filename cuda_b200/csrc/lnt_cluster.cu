@@ -20,6 +20,7 @@
 #include <map>
 
 #include "carry.cuh"
+#include "cluster_exchange.h"
 #include "lazy_core.cuh"
 #include "lnt_internal.h"
 #include "smem_passes.cuh"
@@ -58,12 +59,19 @@ __device__ __forceinline__ void send(const void* local, const uint64_t* bar, uin
 __device__ __forceinline__ void expect_bytes(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
-// Every thread of the CTA waits for the barrier's phase, at most two seconds (an exchange takes under
-// a microsecond).  A wait that gives up is reported and the loop runs on without waiting: every CTA
-// still reaches the end.
-__device__ __forceinline__ void await_phase(uint64_t* bar, uint32_t parity, uint32_t& status) {
+// takes bytes that will not be sent off the barrier's count
+__device__ __forceinline__ void complete_bytes(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void store_remote(const void* local, uint32_t rank, uint64_t v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote_addr(smem_addr(local), rank)), "l"(v) : "memory");
+}
+// Every thread of the CTA waits for the barrier's phase, at most wait_ns (kClusterWaitNs, two seconds:
+// an exchange takes under a microsecond).  A wait that gives up raises kStatusClusterTimeout, and at its
+// next barrier the whole CTA leaves the loop (gave_up); the CTAs that then miss its words give up in turn.
+__device__ __forceinline__ void await_phase(uint64_t* bar, uint32_t parity, const uint64_t& wait_ns, uint32_t& status) {
   uint64_t start = 0;
-  for (uint32_t i = 1; !(status & kStatusFuseTimeout); ++i) {
+  for (uint32_t i = 1; !(status & kStatusClusterTimeout); ++i) {
     uint32_t done;
     asm volatile("{\n\t"
                  ".reg .pred p;\n\t"
@@ -78,10 +86,12 @@ __device__ __forceinline__ void await_phase(uint64_t* bar, uint32_t parity, uint
       uint64_t now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (!start) start = now;
-      if (now - start > 2000000000ull) status |= kStatusFuseTimeout;
+      if (now - start > wait_ns) status |= kStatusClusterTimeout;
     }
   }
 }
+// a barrier of the CTA that also tells whether a wait of any of its threads gave up
+__device__ __forceinline__ bool gave_up(uint32_t status) { return __syncthreads_or((int)(status & kStatusClusterTimeout)) != 0; }
 
 __device__ __forceinline__ int brev_bits(int i, int bits) { return bits ? (int)(__brev((unsigned)i) >> (32 - bits)) : 0; }
 
@@ -89,7 +99,8 @@ __device__ __forceinline__ int brev_bits(int i, int bits) { return bits ? (int)(
 struct Layout {
   uint64_t *a, *b, *w, *uw, *tf0, *ti0, *tf, *ti;
   int64_t *runc, *bc;
-  uint64_t* bar;  // mbarriers: blocks, segments and boundary carries complete
+  uint64_t* bar;   // mbarriers: blocks, segments and boundary carries complete
+  uint64_t* sent;  // exchanges that each CTA sent, at the end
   uint8_t* wd;
 };
 
@@ -97,7 +108,7 @@ constexpr int kMinRun = 4;
 
 __host__ __device__ inline size_t cluster_smem_words(int m, int C) {
   return 4 * (size_t)padded(m) + 2 * (size_t)m /* first pass */ + 2 * (size_t)m /* local passes */ +
-         (size_t)m / kMinRun + (size_t)C + 3 + ((size_t)m + 7) / 8;
+         (size_t)m / kMinRun + 2 * (size_t)C + 3 + ((size_t)m + 7) / 8;
 }
 
 // One pass of the length-m transform on the block buffer.  Mode 0: forward, 1: inverse, 2: last
@@ -187,7 +198,8 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
   S.runc = reinterpret_cast<int64_t*>(S.ti + m);
   S.bc = S.runc + m / kMinRun;
   S.bar = reinterpret_cast<uint64_t*>(S.bc + C);
-  S.wd = reinterpret_cast<uint8_t*>(S.bar + 3);
+  S.sent = S.bar + 3;
+  S.wd = reinterpret_cast<uint8_t*>(S.sent + C);
   if (tid == 0) {
     for (int k = 0; k < 3; ++k)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(S.bar + k)) : "memory");
@@ -256,6 +268,9 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
   // pending carry is read before one is cleared at the end
   cluster_sync();
 
+  // exchanges that this CTA sent, and that it received and re-armed, when it leaves the loop
+  uint64_t sent = 0, passed = 0;
+  bool lost = false;  // this CTA gave up
   for (uint64_t it = 0; it < D.iterations; ++it) {
     const bool um = D.unsigned_first && it == 0;
     // carry-in of the run before, then weight
@@ -268,7 +283,13 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
         v = lazy::mul_digit((int64_t)v, S.w[sw(i * K + k)]);
       }
     }
-    __syncthreads();
+    if (rank == 0 && it == D.quit_at) status |= kStatusClusterTimeout;
+    if ((lost = gave_up(status))) {
+      sent = 3 * it;
+      passed = it ? sent - 1 : 0;
+      break;
+    }
+    if (it && tid == 0) expect_bytes(S.bar + 2, 8u * (uint32_t)C);
     // radix-C pass: block r goes to CTA r
     for (int u = tid; u < seg; u += bd) {
       uint64_t v[C];
@@ -282,15 +303,21 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
       for (int r = 0; r < C; ++r) send(S.b + sw((int)rank * seg + u), S.bar, (uint32_t)r, v[r]);
     }
     const uint32_t parity = (uint32_t)it & 1u;
-    await_phase(S.bar, parity, status);
-    if (tid == 0) expect_bytes(S.bar, 8u * (uint32_t)m);
+    await_phase(S.bar, parity, D.wait_ns, status);
     int span = m, o = 0;
-    for (int j = 0; j + 1 < P.m; ++j) {
+    for (int j = 0; j + 1 < P.m && !lost; ++j) {
       local_pass<0>(P.radix[j], S, m, span, S.tf + o, rank, seg);
       o += span - span / P.radix[j];
       span /= P.radix[j];
-      __syncthreads();
+      if (j) __syncthreads();
+      else lost = gave_up(status);
     }
+    if (lost) {
+      sent = 3 * it + 1;
+      passed = 3 * it;
+      break;
+    }
+    if (tid == 0) expect_bytes(S.bar, 8u * (uint32_t)m);
     local_pass<2>(P.radix[P.m - 1], S, m, span, nullptr, rank, seg);
     __syncthreads();
     for (int j = P.m - 2; j > 0; --j) {
@@ -300,8 +327,7 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
       __syncthreads();
     }
     local_pass<3>(P.radix[0], S, m, m, S.ti, rank, seg);
-    await_phase(S.bar + 1, parity, status);
-    if (tid == 0) expect_bytes(S.bar + 1, 8u * (uint32_t)m);
+    await_phase(S.bar + 1, parity, D.wait_ns, status);
     // inverse radix-C pass, in place on the segments
     for (int u = tid; u < seg; u += bd) {
       uint64_t v[C];
@@ -313,7 +339,12 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
 #pragma unroll
       for (int k = 0; k < C; ++k) S.a[sw(k * seg + u)] = v[k];
     }
-    __syncthreads();
+    if ((lost = gave_up(status))) {
+      sent = 3 * it + 2;
+      passed = 3 * it + 1;
+      break;
+    }
+    if (tid == 0) expect_bytes(S.bar + 1, 8u * (uint32_t)m);
     // unweight and carry; a segment's last carry goes to the CTA that holds the next word
     for (int i = tid; i < runs; i += bd) {
       int64_t carry = (!D.prp && rank == 0 && i == 0) ? -2 : 0;
@@ -332,20 +363,37 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
       }
     }
     __syncthreads();  // the CTA's own run carries
-    await_phase(S.bar + 2, parity, status);
-    if (tid == 0) expect_bytes(S.bar + 2, 8u * (uint32_t)C);
+    await_phase(S.bar + 2, parity, D.wait_ns, status);
+  }
+  if (!lost) {
+    lost = gave_up(status);
+    sent = 3 * D.iterations;
+    passed = lost ? sent - 1 : sent;
   }
 
-  for (int i = tid; i < runs; i += bd) {
-    const int64_t carry = (i & ((1 << lrps) - 1)) ? S.runc[i - 1] : S.bc[i >> lrps];
-    carry_into_run(S.a, S.wd, i * K, K, carry, status);
-    for (int k = 0; k < K; ++k) D.digits[word(i * K + k)] = (int64_t)S.a[sw(i * K + k)];
+  if (!lost) {
+    for (int i = tid; i < runs; i += bd) {
+      const int64_t carry = (i & ((1 << lrps) - 1)) ? S.runc[i - 1] : S.bc[i >> lrps];
+      carry_into_run(S.a, S.wd, i * K, K, carry, status);
+      for (int k = 0; k < K; ++k) D.digits[word(i * K + k)] = (int64_t)S.a[sw(i * K + k)];
+    }
+    if (D.carry)
+      for (int i = tid; i < m / (int)D.tile; i += bd) D.carry[(size_t)rank * (m / (int)D.tile) + i] = 0;
   }
-  if (D.carry)
-    for (int i = tid; i < m / (int)D.tile; i += bd) D.carry[(size_t)rank * (m / (int)D.tile) + i] = 0;
   if (status) atomicOr(D.status, status);
-  // no CTA leaves while another may still be sending to it (a wait that gave up)
+  // No CTA leaves while another may still store into its memory: past this barrier nothing more is
+  // sent, and a CTA that gave up waits (with a limit) for the words on their way to it.  One that did
+  // not give up has received all that was sent to it.
+  if (tid < C) store_remote(S.sent + rank, (uint32_t)tid, sent);
   cluster_sync();
+  if (lost && tid == 0) {
+    for (int b = 0; b < 3; ++b) {
+      const uint32_t missing = cluster::bytes_missing(b, passed, S.sent, rank, C, (uint32_t)m);
+      if (missing) complete_bytes(S.bar + b, missing);
+      uint32_t closing = 0;
+      await_phase(S.bar + b, (uint32_t)(cluster::armed(passed, b) - 1) & 1u, D.wait_ns, closing);
+    }
+  }
 }
 
 template <int C>

@@ -13,6 +13,7 @@ enum : uint32_t {
   kStatusCarryOverflow = 1u << 0,  // a run absorbed a carry above kAbsorbLimit
   kStatusCanonFallback = 1u << 1,  // canonical readout needs the host fallback
   kStatusFuseTimeout = 1u << 2,    // a carry-fused column CTA gave up waiting for its neighbour
+  kStatusClusterTimeout = 1u << 3,  // a CTA of the cluster kernel gave up waiting for words of another
 };
 
 // ---------------------------------------------------------------- plans ----
@@ -129,8 +130,11 @@ struct ClusterDesc {
   uint32_t unsigned_first;  // as ResidentDesc
   uint32_t short_runs;
   uint32_t n1, n2, tile, ntiles;  // run geometry when carry != nullptr
+  uint64_t wait_ns;               // limit of every wait
+  uint64_t quit_at;               // the first CTA leaves before this squaring (lnt_debug_cluster_quit); ~0: never
 };
 constexpr uint32_t kClusterMinLog2 = 9, kClusterMaxLog2 = 15;
+constexpr uint64_t kClusterWaitNs = 2000000000ull;
 
 // CTAs per cluster (0: none), threads per CTA and log2 of the local passes' largest radix for
 // `count` tests of min_n to max_n words in one launch

@@ -232,6 +232,14 @@ int lnt_debug_corrupt(lnt_test* t, uint32_t word);
  * raise the kernels' carry flag, which the check also treats as an error. */
 int lnt_debug_corrupt_add(lnt_test* t, uint32_t word, int64_t delta);
 
+/* Diagnostic without a reference counterpart, for tests of failure detection: in
+ * later launches of the cluster kernel for this test the first CTA leaves before
+ * squaring `squaring` (from 0, of the launch), as if a wait had given up, and no
+ * wait lasts longer than `wait_ns` (at most 2 s).  The other CTAs then give up in turn
+ * and the next readout reports LNT_ERR_CUDA.  LNT_ERR_UNSUPPORTED_LENGTH for a
+ * test that does not run on the cluster kernel. */
+int lnt_debug_cluster_quit(lnt_test* t, uint64_t squaring, uint64_t wait_ns);
+
 /* Length, widths (n bytes: ceil(q(j+1)/n) - ceil(qj/n), pre_calculation.cu:35
  * in exact integers) and plan name of a test. */
 int lnt_get_length(lnt_test* t, uint32_t* n);

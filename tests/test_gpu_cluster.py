@@ -83,3 +83,28 @@ def test_two_pass_groups_take_over(lnt):
         with lnt.LucasTest(q, prp=True) as t:
             t.iterate(50)
             assert got[i] == t.res64()
+
+
+@pytest.mark.parametrize("q,n", [(9689, 512), (44021, 2048), (160001, 8192), (620009, 32768)])
+@pytest.mark.parametrize("squaring", [0, 1, 6])
+def test_a_wait_that_gives_up(lnt, oracle_mod, q, n, squaring):
+    """A CTA that leaves early: the others give up at waits of 50 ms, the readout reports it, and
+    the GPU runs on.  A launch that ends before that squaring is not touched."""
+    start = random_digits(q, n, q + 1)
+    with lnt.LucasTest(q, n, True) as t:
+        t.set_digits(start)
+        if squaring:
+            t.debug_cluster_quit(squaring)
+            t.iterate(squaring)
+            t.synchronize()
+        t.debug_cluster_quit(squaring)
+        t.iterate(20)
+        with pytest.raises(lnt.LucasNTTError, match="cluster kernel timed out") as e:
+            t.digits()
+        assert e.value.status == 3
+    with lnt.LucasTest(q, n, True) as t, oracle_mod.OracleTest(q, n, True) as o:
+        t.set_digits(start)
+        o.set_digits(start)
+        t.iterate(4)
+        o.iterate(4)
+        assert np.array_equal(t.digits(), o.digits())
