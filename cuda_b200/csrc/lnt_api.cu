@@ -52,7 +52,7 @@ struct lnt_test {
   uint64_t *tw5 = nullptr, *itw5 = nullptr;  // n = 5 * 2^k: the radix-5 step's twiddles
   uint64_t c5[4] = {};                        // and its constants
   uint64_t cluster_wait_ns = lnt::kClusterWaitNs, cluster_quit_at = ~0ull;  // lnt_debug_cluster_quit
-  uint64_t* pw = nullptr;  // omega_n^e of the cluster kernel (512 ... 32768 words, policy plans)
+  uint64_t* pw = nullptr;  // omega_n^e of the cluster kernel, or nullptr: the test does not run on it alone
   // separable weights of the register-pass column kernels (TwoPassDesc)
   ulonglong2 *rowf = nullptr, *colw = nullptr;
   uint32_t* colf = nullptr;
@@ -163,16 +163,19 @@ void pass_table(uint32_t n, uint32_t max_radix, bool inverse, std::vector<uint64
   power_table(n, inverse, pw);
   const std::vector<uint32_t> radix = lnt::r16_pass_radices(log2n, max_radix);
   out.clear();
+  out.reserve((size_t)n * 3 / 2);
   uint32_t span = n;
   for (size_t j = 0; j + 1 < radix.size(); ++j) {
     const uint32_t R = radix[j], q = span / R, scale = n / span;
     uint32_t bits = 0;
     while ((1u << bits) < R) ++bits;
-    for (uint32_t i = 0; i < span; ++i) {
-      const uint32_t t = i / 2 % q, r = i / (2 * q) * 2 + i % 2;
-      uint32_t b = 0;
-      for (uint32_t k = 0; k < bits; ++k) b |= ((r >> k) & 1u) << (bits - 1 - k);
-      out.push_back(pw[(size_t)t * b * scale]);
+    for (uint32_t pair = 0; pair < R / 2; ++pair) {
+      size_t step[2] = {0, 0};  // brev_R(r) of the pair's two elements
+      for (uint32_t k = 0; k < bits; ++k)
+        for (uint32_t i = 0; i < 2; ++i)
+          step[i] |= (size_t)(((2 * pair + i) >> k) & 1u) << (bits - 1 - k);
+      for (uint32_t t = 0; t < q; ++t)
+        for (uint32_t i = 0; i < 2; ++i) out.push_back(pw[t * step[i] * scale]);
     }
     span /= R;
   }
@@ -435,9 +438,22 @@ void capture_graph(lnt_test* t, const lnt::TwoPassDesc& d) {
   if (!t->graph) t->graph_failed = true;
 }
 
-// Policy plans of 512 to 32768 words also run on the cluster kernel.
+// Policy plans of 512 to 32768 words can also run on the cluster kernel; a test that has its table of
+// powers (make_powers) does.
 bool cluster_plan(const lnt::Plan& p) {
   return p.policy && !p.five && p.log2n >= lnt::kClusterMinLog2 && p.log2n <= lnt::kClusterMaxLog2;
+}
+
+cudaError_t make_powers(lnt_test* t, cudaStream_t s) {
+  if (t->pw) return cudaSuccess;
+  cudaError_t e = dalloc(&t->pw, t->n);
+  if (e == cudaSuccess) e = lnt::launch_powers(t->n, t->pw, s);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (t->pw) cudaFree(t->pw);
+    t->pw = nullptr;
+  }
+  return e;
 }
 
 lnt::ClusterDesc cluster_desc(const lnt_test* t, uint64_t iterations) {
@@ -470,7 +486,7 @@ lnt::ClusterDesc cluster_desc(const lnt_test* t, uint64_t iterations) {
 }
 
 int queue_iterations(lnt_test* t, uint64_t iterations, LaunchTimer* timer) {
-  const lnt::ClusterChoice cl = cluster_plan(t->plan) ? lnt::cluster_choice(t->n, t->n, 1) : lnt::ClusterChoice();
+  const lnt::ClusterChoice cl = t->pw ? lnt::cluster_choice(t->n, t->n, 1) : lnt::ClusterChoice();
   if (cl.size) {
     const lnt::ClusterDesc d = cluster_desc(t, iterations);
     LNT_LAUNCH(lnt::launch_cluster(nullptr, d, 1, t->n, cl.size, cl.threads, cl.pass_log2, t->stream),
@@ -999,6 +1015,8 @@ ResidentDesc test_resident_desc(const lnt_test* t, uint64_t iterations) {
   return d;
 }
 ClusterDesc test_cluster_desc(const lnt_test* t, uint64_t iterations) { return cluster_desc(t, iterations); }
+bool test_cluster_plan(const lnt_test* t) { return cluster_plan(t->plan); }
+cudaError_t test_make_powers(lnt_test* t, cudaStream_t s) { return make_powers(t, s); }
 // bookkeeping after squarings were launched outside lnt_iterate
 void test_mark_iterated(lnt_test* t) {
   if (t->plan.kind == PlanKind::TwoPass) t->pending_carries = true;
@@ -1069,6 +1087,13 @@ int lnt_create(uint32_t exponent, uint32_t n, int prp, int device, lnt_test** ou
 
 int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
                          const lnt_plan_options* options, lnt_test** out) {
+  return lnt::create_test(exponent, n, prp, device, options, true, out);
+}
+
+}  // extern "C"
+
+int lnt::create_test(uint32_t exponent, uint32_t n, int prp, int device, const lnt_plan_options* options, bool alone,
+                     lnt_test** out) {
   if (!out) return fail(LNT_ERR_INVALID_ARGUMENT, "null output pointer");
   *out = nullptr;
   if (exponent < 3) return fail(LNT_ERR_INVALID_ARGUMENT, "exponent must be >= 3");
@@ -1124,14 +1149,7 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
     return bail(cuda_fail(e, "weights"));
 
   int st;
-  std::vector<uint64_t> powers;
-  if (cluster_plan(plan)) {
-    power_table(n, false, powers);
-    if ((e = dalloc(&t->pw, n)) ||
-        (e = cudaMemcpyAsync(t->pw, powers.data(), (size_t)n * 8, cudaMemcpyHostToDevice, t->stream)) ||
-        (e = cudaStreamSynchronize(t->stream)))
-      return bail(cuda_fail(e, "powers"));
-  }
+  if (alone && cluster_plan(plan) && (e = make_powers(t, t->stream))) return bail(cuda_fail(e, "powers"));
   if (plan.kind == lnt::PlanKind::Resident) {
     if ((st = upload_roots(t, n, &t->rt, &t->irt, 8)) != LNT_OK) return bail(st);  // the resident kernel's passes
     if ((e = dalloc(&t->rdesc, 1))) return bail(cuda_fail(e, "allocate descriptor"));
@@ -1184,6 +1202,8 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
   *out = t;
   return LNT_OK;
 }
+
+extern "C" {
 
 int lnt_destroy(lnt_test* t) {
   if (!t) return LNT_OK;

@@ -532,7 +532,7 @@ int admit(lnt_batch* b, uint64_t id, uint32_t exponent, uint32_t n, int prp, uin
     }
     plan = &it->second;
   }
-  st = lnt_create_with_plan(exponent, n, prp, b->device, plan, &t);
+  st = lnt::create_test(exponent, n, prp, b->device, plan, false, &t);
   if (st != LNT_OK) return st;
   Entry e{};
   e.id = id;
@@ -681,15 +681,21 @@ int lnt_batch_run(lnt_batch* b, uint64_t iterations) {
       if (budget)
         step[i] = std::min<uint64_t>(step[i], std::max<uint64_t>(1, (uint64_t)(b->step_seconds / (rate * e.n))));
       h.push_back(lnt::test_resident_desc(e.t, step[i]));
-      hc.push_back(lnt::test_cluster_desc(e.t, step[i]));
       max_n = std::max(max_n, e.n);
       min_n = std::min(min_n, e.n);
       resident_work = std::max<uint64_t>(resident_work, step[i] * e.n);
     }
-    // few tests: each over a cluster of CTAs; else one CTA per test
+    // few tests: each over a cluster of CTAs (whose tables are made now, when one is first launched);
+    // else one CTA per test
     lnt::ClusterChoice cl;
-    if (std::all_of(hc.begin(), hc.end(), [](const lnt::ClusterDesc& d) { return d.pw != nullptr; }))
+    if (std::all_of(b->resident.begin(), b->resident.end(),
+                    [&](size_t i) { return lnt::test_cluster_plan(b->active[i].t); }))
       cl = lnt::cluster_choice(min_n, max_n, (uint32_t)h.size());
+    for (size_t k = 0; k < b->resident.size() && cl.size; ++k) {
+      const size_t i = b->resident[k];
+      if (lnt::test_make_powers(b->active[i].t, b->rstream) != cudaSuccess) cl = lnt::ClusterChoice();
+      else hc.push_back(lnt::test_cluster_desc(b->active[i].t, step[i]));
+    }
     if (cl.size) {
       BCUDA(cudaMemcpyAsync(b->d_cdescs, hc.data(), hc.size() * sizeof(lnt::ClusterDesc),
                             cudaMemcpyHostToDevice, b->rstream),

@@ -230,6 +230,8 @@ cudaError_t launch_col_fused_r16(const TwoPassDesc& d, const TwoPassDesc* dd, ui
                                  cudaStream_t s);
 
 // ------------------------------------------------------------- tables ----
+// omega_n^e, e < n (the cluster kernel's table)
+cudaError_t launch_powers(uint32_t n, uint64_t* pw, cudaStream_t s);
 cudaError_t launch_weights(uint32_t exponent, uint32_t n, uint64_t* w, uint64_t* uw,
                            cudaStream_t s);
 // colw == nullptr: plain twiddles; else colw[j1] = {g^fa / 2, g^-fa} multiplied in
@@ -270,6 +272,7 @@ cudaError_t launch_fill_max(uint64_t* out, const uint8_t* widths, uint32_t n, cu
 }  // namespace lnt
 
 struct lnt_test;
+struct lnt_plan_options;
 
 namespace lnt {
 const Plan& test_plan(const lnt_test* t);
@@ -279,6 +282,13 @@ TwoPassDesc test_twopass_desc(const lnt_test* t);
 bool test_ready_for_group(const lnt_test* t);
 ResidentDesc test_resident_desc(const lnt_test* t, uint64_t iterations);
 ClusterDesc test_cluster_desc(const lnt_test* t, uint64_t iterations);
+// may run on the cluster kernel, given the table of powers that test_make_powers queues on `s`
+bool test_cluster_plan(const lnt_test* t);
+cudaError_t test_make_powers(lnt_test* t, cudaStream_t s);
+// lnt_create_with_plan; `alone`: squarings run one test at a time.  The batch's tests are made without it:
+// most of them never see the cluster kernel, and 160 of them spent 4 ms of 28 ms on tables for it.
+int create_test(uint32_t exponent, uint32_t n, int prp, int device, const lnt_plan_options* options, bool alone,
+                lnt_test** out);
 void test_mark_iterated(lnt_test* t);
 uint64_t test_device_bytes(uint32_t n);
 void set_last_error(const std::string& msg);

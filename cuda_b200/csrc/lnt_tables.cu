@@ -91,6 +91,18 @@ cudaError_t launch_weight_factors(uint32_t exponent, uint32_t n1, uint32_t n2, u
   return cudaGetLastError();
 }
 
+namespace {
+__global__ void power_kernel(uint32_t n, uint64_t root, uint64_t* pw) {
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < n) pw[e] = gl::pow(root, e);
+}
+}  // namespace
+
+cudaError_t launch_powers(uint32_t n, uint64_t* pw, cudaStream_t s) {
+  power_kernel<<<(n + 127) / 128, 128, 0, s>>>(n, gl::pow(554, (gl::P - 1) / n), pw);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_weights(uint32_t exponent, uint32_t n, uint64_t* w, uint64_t* uw,
                            cudaStream_t s) {
   const uint64_t c = ((gl::P - 1) / 192 / n) * 5ull;

@@ -252,3 +252,21 @@ def test_time_budgeted_calls_equal_alone(lnt):
     for i, (q, n, prp, k) in ids.items():
         assert got[i]["status"] == 0 and got[i]["res64"] == alone(lnt, q, n, prp, k), (q, prp)
     assert calls[9941] < calls[12000017], calls
+
+
+def test_admission_makes_no_tables_for_kernels_it_does_not_run(lnt):
+    """128 tests of 32768 words, which run in a group of the two-pass kernels: the memory they take
+    leaves out the cluster kernel's table (8 bytes of about 43 a word)."""
+    import torch
+
+    tests, n, q = 128, 32768, 620009
+    per_test = lnt.lib().lnt_test_device_bytes(q, n)
+    with lnt.Batch() as b:
+        b.submit(q, n=n, prp=True, iterations=2)  # kernels loaded, first blocks reserved
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        for _ in range(tests):
+            b.submit(q, n=n, prp=True, iterations=2)
+        torch.cuda.synchronize()
+        taken = before - torch.cuda.mem_get_info()[0]
+    assert taken < tests * (per_test - 4 * n), (taken / tests / n, per_test / n)

@@ -74,7 +74,8 @@ def test_batches_of_every_cluster_size(lnt, count):
 
 
 def test_two_pass_groups_take_over(lnt):
-    """A batch admits a test with one squaring on the cluster kernel, then runs it in its group."""
+    """Batches of 8K words and more run on the two-pass kernels from the first squaring on, and end on
+    the residues that the cluster kernel gives."""
     with lnt.Batch() as b:
         ids = [b.submit(q, prp=True, iterations=50) for q in (160001, 160033, 316003)]
         b.run(50)
