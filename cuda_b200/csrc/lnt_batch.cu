@@ -63,7 +63,7 @@ struct Pending {
 };
 
 // Tests share launches when their kernels see the same geometry: length,
-// split, tile, pass radix (the pass tables differ) and column fusion.
+// split, tile, pass radix (the pass tables differ where it makes a difference) and column fusion.
 struct GroupKey {
   uint32_t n, log2n2, tile, radix;
   bool fused;
@@ -266,7 +266,7 @@ int rebuild(lnt_batch* b) {
       b->resident.push_back(i);
     } else if (p.fast && lnt::test_ready_for_group(b->active[i].t)) {
       // one launch serves tests of identical geometry
-      Group& g = b->groups[GroupKey{p.n, p.log2n2, p.tile, p.radix, p.fused}];
+      Group& g = b->groups[GroupKey{p.n, p.log2n2, p.tile, lnt::r16_plan_radix(p.radix, p.five, p.n1, p.n2), p.fused}];
       g.n = p.n;
       g.fused = p.fused;
       g.members.push_back(i);

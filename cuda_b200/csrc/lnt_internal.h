@@ -208,6 +208,10 @@ std::vector<uint32_t> r16_pass_radices(uint32_t log2L, uint32_t radix);
 // in launches of few CTAs (8 in larger ones); lnt_radix16.cu says where the lines lie.
 uint32_t r16_row_radix(uint32_t plan_radix, uint32_t n1);
 uint32_t r16_col_radix(uint32_t plan_radix, bool five, uint32_t n2);
+// Plans that differ in their radix alone run the same kernels where this is the same.
+inline uint32_t r16_plan_radix(uint32_t plan_radix, bool five, uint32_t n1, uint32_t n2) {
+  return r16_row_radix(plan_radix, n1) == 16 || r16_col_radix(plan_radix, five, n2) == 16 ? 16 : 8;
+}
 uint32_t r16_tile(uint32_t log2n2);
 uint32_t r16_run_words_needed(uint32_t exponent, uint32_t n);
 // `d` gives the geometry (shared by every test of the launch); `dd` is a device

@@ -305,6 +305,8 @@ std::vector<PlanOptions> plan_candidates(uint32_t n, uint32_t exponent) {
           if (!make_plan(n, exponent, &o, p)) continue;
           const int skew = (int)p.log2n1 - (int)p.log2n2;
           if (!r16 && (skew < 0 || skew > 3)) continue;
+          // radix 16 that takes 16 points nowhere is radix 8 by another name
+          if (p.fast && !p.five && p.radix != r16_plan_radix(p.radix, false, p.n1, p.n2)) continue;
           add(o);
         }
   return out;

@@ -118,6 +118,18 @@ def test_smallest_length(lnt):
     assert lnt.smallest_length(170000009) == 5 << 21 and lnt.smallest_length(139000003) == 1 << 23
 
 
+def test_candidates_run_different_kernels(lnt):
+    """A radix-16 plan is listed only where it takes 16-point passes: columns of 1024 words and
+    more, or rows of 1024 or 2048 words."""
+    for k in range(13, 27):
+        plans = lnt.plan_candidates(14 << k, 1 << k)
+        assert len(set(plans)) == len(plans)
+        for kind, log2_rows, tile, radix, fused in plans:
+            n2, n1 = 1 << log2_rows, (1 << k) >> log2_rows
+            assert radix == 8 or n2 >= 1024 or n1 in (1024, 2048), (k, log2_rows)
+        assert any(p[3] == 16 for p in plans) == (k >= 16), k
+
+
 def test_five_length_plans_at_every_k(lnt):
     """Every 5 * 2^k length, 13 <= k <= 24, has register-pass plans only (radix
     8), rows of 5 L words with 2^7 <= L <= 2^12 and columns 2^6 ... 2^12; the
