@@ -1481,6 +1481,18 @@ int lnt_plan_describe(const lnt_plan_options* o, uint32_t exponent, uint32_t n, 
 // events on its stream; the fastest wins.
 int lnt_time_plans(uint32_t exponent, uint32_t n, int prp, int device, uint32_t loops,
                    const lnt_plan_options* plans, int count, float* ms) {
+  return lnt::time_plans(exponent, n, prp, device, loops, plans, count, ms, true);
+}
+
+int lnt_autotune(uint32_t exponent, uint32_t n, int prp, int device, uint32_t loops,
+                 lnt_plan_options* tried, float* ms, int cap, int* count, int* best) {
+  return lnt::autotune(exponent, n, prp, device, loops, tried, ms, cap, count, best, true);
+}
+
+}  // extern "C"
+
+int lnt::time_plans(uint32_t exponent, uint32_t n, int prp, int device, uint32_t loops, const lnt_plan_options* plans,
+                    int count, float* ms, bool alone) {
   if ((count > 0 && (!plans || !ms)) || count < 0) return fail(LNT_ERR_INVALID_ARGUMENT, "null argument");
   if (loops == 0) return fail(LNT_ERR_INVALID_ARGUMENT, "loops must be > 0");
   if (n == 0) n = 1u << lnt_secured_log2_length(exponent);
@@ -1488,7 +1500,7 @@ int lnt_time_plans(uint32_t exponent, uint32_t n, int prp, int device, uint32_t 
   for (int i = 0; i < count; ++i) {
     lnt_test* t = nullptr;
     float elapsed = -1;
-    int st = lnt_create_with_plan(exponent, n, prp, device, &plans[i], &t);
+    int st = create_test(exponent, n, prp, device, &plans[i], alone, &t);
     if (st == LNT_OK) {
       DeviceGuard guard(t->device);
       cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1517,8 +1529,8 @@ int lnt_time_plans(uint32_t exponent, uint32_t n, int prp, int device, uint32_t 
   return ok ? LNT_OK : last_status;
 }
 
-int lnt_autotune(uint32_t exponent, uint32_t n, int prp, int device, uint32_t loops,
-                 lnt_plan_options* tried, float* ms, int cap, int* count, int* best) {
+int lnt::autotune(uint32_t exponent, uint32_t n, int prp, int device, uint32_t loops, lnt_plan_options* tried, float* ms,
+                  int cap, int* count, int* best, bool alone) {
   if (!count || !best || (cap > 0 && (!tried || !ms))) return fail(LNT_ERR_INVALID_ARGUMENT, "null argument");
   if (n == 0) n = 1u << lnt_secured_log2_length(exponent);
   const std::vector<lnt::PlanOptions> c = lnt::plan_candidates(n, exponent);
@@ -1527,7 +1539,7 @@ int lnt_autotune(uint32_t exponent, uint32_t n, int prp, int device, uint32_t lo
   std::vector<float> t(plans.size(), -1.0f);
   *count = (int)plans.size();
   *best = -1;
-  const int st = lnt_time_plans(exponent, n, prp, device, loops, plans.data(), (int)plans.size(), t.data());
+  const int st = time_plans(exponent, n, prp, device, loops, plans.data(), (int)plans.size(), t.data(), alone);
   for (size_t i = 0; i < plans.size(); ++i) {
     if ((int)i < cap) {
       tried[i] = plans[i];
@@ -1538,6 +1550,8 @@ int lnt_autotune(uint32_t exponent, uint32_t n, int prp, int device, uint32_t lo
   if (plans.empty()) return fail(LNT_ERR_UNSUPPORTED_LENGTH, "no plan for this length");
   return st;
 }
+
+extern "C" {
 
 // LucasPRP::DumpEnvironment (lucas_prp.cu:265-291): the same lines, for the
 // host program, which has no CUDA headers of its own.

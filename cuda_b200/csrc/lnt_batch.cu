@@ -520,7 +520,8 @@ int admit(lnt_batch* b, uint64_t id, uint32_t exponent, uint32_t n, int prp, uin
         lnt_plan_options tried[128];
         float ms[128];
         int count = 0, best = -1;
-        st = lnt_autotune(exponent, n, prp, b->device, b->tune_loops, tried, ms, 128, &count, &best);
+        // one test, on the kernels that its group will run
+        st = lnt::autotune(exponent, n, prp, b->device, b->tune_loops, tried, ms, 128, &count, &best, false);
         if (st == LNT_OK && best >= 0 && best < 128) {
           chosen = tried[best];
           best_ms = ms[best];

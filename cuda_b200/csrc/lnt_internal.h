@@ -293,6 +293,11 @@ cudaError_t test_make_powers(lnt_test* t, cudaStream_t s);
 // most of them never see the cluster kernel, and 160 of them spent 4 ms of 28 ms on tables for it.
 int create_test(uint32_t exponent, uint32_t n, int prp, int device, const lnt_plan_options* options, bool alone,
                 lnt_test** out);
+// lnt_time_plans and lnt_autotune on the kernels that a test made so runs on
+int time_plans(uint32_t exponent, uint32_t n, int prp, int device, uint32_t loops, const lnt_plan_options* plans,
+               int count, float* ms, bool alone);
+int autotune(uint32_t exponent, uint32_t n, int prp, int device, uint32_t loops, lnt_plan_options* tried, float* ms,
+             int cap, int* count, int* best, bool alone);
 void test_mark_iterated(lnt_test* t);
 uint64_t test_device_bytes(uint32_t n);
 void set_last_error(const std::string& msg);

@@ -270,3 +270,16 @@ def test_admission_makes_no_tables_for_kernels_it_does_not_run(lnt):
         torch.cuda.synchronize()
         taken = before - torch.cuda.mem_get_info()[0]
     assert taken < tests * (per_test - 4 * n), (taken / tests / n, per_test / n)
+
+
+def test_batch_autotune_times_the_kernels_of_the_group(lnt, tmp_path):
+    """At 8192 words a lone test runs on the cluster kernel (7 us a squaring), a batch on the
+    two-pass kernels (15 us): the batch's plan is chosen by the time of the latter."""
+    import json
+
+    path, loops, q = tmp_path / "plans.json", 200, 160001
+    lone, best = lnt.autotune(q, 8192, True, 0, loops)
+    with lnt.Batch(device=0, autotune_loops=loops, plan_cache=str(path)) as b:
+        b.submit(q, 8192, True, 10)
+    tuned = json.loads(path.read_text())["plans"][0]
+    assert tuned["n"] == 8192 and tuned["ms"] > 1.4 * lone[best][1]
