@@ -37,6 +37,7 @@
 #include <vector>
 
 #include "../../include/lucasntt.h"
+#include "grow_array.h"
 #include "lnt_internal.h"
 
 namespace {
@@ -112,9 +113,8 @@ struct lnt_batch {
   std::map<GroupKey, Group> groups;  // fast two-pass tests by geometry
   std::vector<size_t> resident;      // SMEM-resident tests
   std::vector<size_t> singles;       // tests iterated one by one
-  lnt::ResidentDesc* d_rdescs = nullptr;
-  size_t rcap = 0;
-  lnt::ClusterDesc* d_cdescs = nullptr;  // the same tests when few enough for the cluster kernel
+  lnt::GrowArray<lnt::ResidentDesc> rdescs;
+  lnt::GrowArray<lnt::ClusterDesc> cdescs;  // the same tests when few enough for the cluster kernel
   std::vector<cudaStream_t> spare_streams;
   cudaStream_t rstream = nullptr;    // the resident launch, beside the groups
   cudaEvent_t fork = nullptr;        // recorded on `stream` before the group launches
@@ -158,6 +158,9 @@ struct DeviceGuard {
     if (e_ != cudaSuccess) return berr(LNT_ERR_CUDA, std::string(what) + ": " +    \
                                                          cudaGetErrorString(e_)); \
   } while (0)
+
+cudaError_t dev_alloc(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
+void dev_free(void* p) { cudaFree(p); }
 
 cudaStream_t take_stream(lnt_batch* b) {
   if (!b->spare_streams.empty()) {
@@ -291,14 +294,8 @@ int rebuild(lnt_batch* b) {
     BCUDA(cudaEventCreate(&g.t0), "group event");
     BCUDA(cudaEventCreate(&g.t1), "group event");
   }
-  if (b->resident.size() > b->rcap) {
-    if (b->d_rdescs) cudaFree(b->d_rdescs);
-    b->rcap = std::max<size_t>(b->resident.size(), 2 * b->rcap);
-    BCUDA(cudaMalloc((void**)&b->d_rdescs, b->rcap * sizeof(lnt::ResidentDesc)), "resident descriptors");
-    if (b->d_cdescs) cudaFree(b->d_cdescs);
-    b->d_cdescs = nullptr;
-    BCUDA(cudaMalloc((void**)&b->d_cdescs, b->rcap * sizeof(lnt::ClusterDesc)), "resident descriptors");
-  }
+  BCUDA(b->rdescs.reserve(b->resident.size(), dev_alloc, dev_free), "resident descriptors");
+  BCUDA(b->cdescs.reserve(b->resident.size(), dev_alloc, dev_free), "resident descriptors");
   b->dirty = false;
   return LNT_OK;
 }
@@ -376,8 +373,8 @@ int lnt_batch_destroy(lnt_batch* b) {
     if (e) cudaEventDestroy(e);
   for (cudaStream_t s : b->spare_streams)
     if (s) cudaStreamDestroy(s);
-  if (b->d_rdescs) cudaFree(b->d_rdescs);
-  if (b->d_cdescs) cudaFree(b->d_cdescs);
+  b->rdescs.clear(dev_free);
+  b->cdescs.clear(dev_free);
   if (b->stream) cudaStreamDestroy(b->stream);
   if (b->rstream) cudaStreamDestroy(b->rstream);
   delete b;
@@ -698,19 +695,19 @@ int lnt_batch_run(lnt_batch* b, uint64_t iterations) {
       else hc.push_back(lnt::test_cluster_desc(b->active[i].t, step[i]));
     }
     if (cl.size) {
-      BCUDA(cudaMemcpyAsync(b->d_cdescs, hc.data(), hc.size() * sizeof(lnt::ClusterDesc),
+      BCUDA(cudaMemcpyAsync(b->cdescs.data, hc.data(), hc.size() * sizeof(lnt::ClusterDesc),
                             cudaMemcpyHostToDevice, b->rstream),
             "upload resident descriptors");
       BCUDA(cudaEventRecord(b->r0, b->rstream), "resident timer");
-      BCUDA(lnt::launch_cluster(b->d_cdescs, hc[0], (uint32_t)hc.size(), max_n, cl.size, cl.threads, cl.pass_log2,
+      BCUDA(lnt::launch_cluster(b->cdescs.data, hc[0], (uint32_t)hc.size(), max_n, cl.size, cl.threads, cl.pass_log2,
                                 b->rstream),
             "cluster kernel");
     } else {
-      BCUDA(cudaMemcpyAsync(b->d_rdescs, h.data(), h.size() * sizeof(lnt::ResidentDesc),
+      BCUDA(cudaMemcpyAsync(b->rdescs.data, h.data(), h.size() * sizeof(lnt::ResidentDesc),
                             cudaMemcpyHostToDevice, b->rstream),
             "upload resident descriptors");
       BCUDA(cudaEventRecord(b->r0, b->rstream), "resident timer");
-      BCUDA(lnt::launch_resident(b->d_rdescs, (uint32_t)h.size(), max_n, b->rstream), "resident kernel");
+      BCUDA(lnt::launch_resident(b->rdescs.data, (uint32_t)h.size(), max_n, b->rstream), "resident kernel");
     }
     BCUDA(cudaEventRecord(b->r1, b->rstream), "resident timer");
   }

@@ -114,3 +114,13 @@ def test_length_queries_reject_bad_arguments(lnt):
     assert L.lnt_shifted_words(100003, 3 << 12, ctypes.byref(c), None) == 1  # not a power of two
     assert L.lnt_shifted_words(100003, 1 << 27, ctypes.byref(c), None) == 1
     assert L.lnt_shifted_words(100003, 1 << 12, ctypes.byref(c), None) == 0 and c.value == 0
+
+
+def test_descriptor_arrays_after_a_failed_allocation(tmp_path):
+    """The batch's descriptor arrays hold nothing after an allocation that failed, and the next call
+    tries again."""
+    exe = tmp_path / "grow_array_selftest"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-o", str(exe),
+                    str(ROOT / "tests" / "native" / "grow_array_selftest.cpp")], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout
