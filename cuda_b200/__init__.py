@@ -11,6 +11,7 @@ from .api import (  # noqa: F401
     arith_selftest,
     autotune,
     check_provided_length,
+    lazy_selftest,
     length_candidates,
     lib,
     parse_length,

@@ -131,6 +131,7 @@ def lib() -> ctypes.CDLL:
         "lnt_batch_poll_checkpoints": ([vp, ctypes.POINTER(BatchCheckpoint), i32, ctypes.POINTER(i32)], i32),
         "lnt_batch_plan_cache": ([vp, cp], i32),
         "lnt_arith_selftest": ([i32, ctypes.POINTER(u64), ctypes.POINTER(u64)], i32),
+        "lnt_lazy_selftest": ([i32, ctypes.POINTER(u64), ctypes.POINTER(u64)], i32),
     }
     for name, (args, res) in sigs.items():
         f = getattr(L, name)
@@ -212,6 +213,14 @@ def arith_selftest(device: int = 0) -> int:
     and raises LucasNTTError (LNT_ERR_NUMERIC) on any mismatch."""
     checked, bad = ctypes.c_uint64(), ctypes.c_uint64()
     _check(lib().lnt_arith_selftest(device, ctypes.byref(checked), ctypes.byref(bad)), "lnt_arith_selftest")
+    return int(checked.value)
+
+
+def lazy_selftest(device: int = 0) -> int:
+    """lnt_lazy_selftest: as arith_selftest, for the lazily reduced products and
+    transforms and the carry steps."""
+    checked, bad = ctypes.c_uint64(), ctypes.c_uint64()
+    _check(lib().lnt_lazy_selftest(device, ctypes.byref(checked), ctypes.byref(bad)), "lnt_lazy_selftest")
     return int(checked.value)
 
 

@@ -267,6 +267,10 @@ int lnt_environment(char* out, size_t outlen);
  * LNT_ERR_NUMERIC (first mismatch in lnt_last_error) if any differs. */
 int lnt_arith_selftest(int device, uint64_t* checked, uint64_t* mismatches);
 
+/* The same for the lazily reduced arithmetic of the kernels: products, register
+ * transforms, digit products, and the digits and carries of the carry steps. */
+int lnt_lazy_selftest(int device, uint64_t* checked, uint64_t* mismatches);
+
 /* Run the test's work on a caller-owned cudaStream_t (NULL = the test's own
  * stream), the analogue of common::stream (common/common.cu:118). */
 int lnt_set_stream(lnt_test* t, void* cuda_stream);

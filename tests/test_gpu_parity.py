@@ -248,3 +248,10 @@ def test_device_arithmetic_against_host(lnt):
     their rare branches and on seeded random operands."""
     checked = lnt.arith_selftest(0)
     assert checked == (25 * 25 + 3 * 8192) * 16
+
+
+def test_device_lazy_arithmetic_against_host(lnt):
+    """The same for the arithmetic of the squaring kernels: lazily reduced products and transforms of
+    2, 4, 5, 8 and 16 points, digit products, and the digits and carries of the carry steps."""
+    checked = lnt.lazy_selftest(0)
+    assert checked == (25 * 25 + 3 * 8192) * 90
