@@ -15,11 +15,18 @@
 // 441.2 us with canonical values and takes 363.1 us with these (row_square 210.5 -> 161.5,
 // col_fused 240.8 -> 212.2); n = 2048 on one SM 10.15 -> 8.99 us.
 //
-// Ranges.  Inputs of a network: |x| < 2^66 (a 64-bit word, or the three words of
-// mul3, in (-2^32, 2^65)).  Differences are then below 2^67, times 2^24 below
-// 2^91, and no sum passes 2^93: three words never overflow.  The bias kBias p
-// (2^28 p, congruent to 0) is added to input 0, which reaches every output with
-// coefficient +1, so every output is non-negative and below 2^93.
+// Ranges.  Inputs of a network: |x| <= 2^65 (a 64-bit word, or the three words of
+// mul3, in (-2^32, 2^65)); a sum of two words is too large.  Then, for 16 points:
+// - a first 4-point step leaves at most 2^67 (s0 +- s1), or 1.5 2^66 + 2^33 where one of its
+//   terms came from mul_2_48 (which leaves 2^65 + 2^33);
+// - times 2^24 that is at most 2^91; the second bound times 2^12, plus a term below 2^66, stays below
+//   the 2^79 that mul_2_48 takes; mul_mid<60>, which takes 2^67, sees the second bound only, and
+//   mul_mid<36>, mul_2_72 and mul_high<84> take 2^75 and more;
+// - at most one term of an output is a multiple of 2^24, so without the bias its magnitude is
+//   below 2^92.
+// Fewer points leave less.  The bias kBias p (2^28 p, congruent to 0) is added to input 0, which
+// reaches every output with coefficient +1 and is never multiplied, so every output is
+// non-negative and below 2^93: three words never overflow.
 //
 // On the host the same formulas run on 128-bit integers and check those ranges
 // (tests/native/lazy_selftest.cpp).
@@ -38,6 +45,9 @@ struct W3 {
 };
 
 constexpr uint32_t kBias = 1u << 28;
+#if !defined(__CUDA_ARCH__)
+constexpr __int128 kInputBound = (__int128)1 << 65;
+#endif
 
 GL_HD W3 from_word(uint64_t x) { return {(uint32_t)x, (uint32_t)(x >> 32), 0u}; }
 
@@ -462,7 +472,7 @@ inline void dft5_constants(uint64_t w, uint64_t c[4]) {
   c[3] = gl::mul(4, gl::add(s1, s2));
 }
 
-// Four times the 5-point transform, |u| < 2^66, in four general products.  With a1, b1 = u1 +- u4
+// Four times the 5-point transform, |u| <= 2^65, in four general products.  With a1, b1 = u1 +- u4
 // and a2, b2 = u2 +- u3 the outputs are u0 + a1 + a2 and u0 + t +- s for (t, s) = (a1 C1 + a2 C2,
 // b1 S1 + b2 S2) and (a1 C2 + a2 C1, b1 S2 - b2 S1).  C1 + C2 = -1/2 leaves one product for both t
 // (4 t = -(a1 + a2) +- 2 (a1 - a2)(C1 - C2)), three make both s.  The inverse transform is the same

@@ -1,7 +1,8 @@
 // Host check of the lazily reduced transforms (cuda_b200/csrc/lazy_core.cuh): dif<R> and
 // dit_inv<R> on any 64-bit words, and on products of such words, are congruent to the
 // canonical transforms (ntt_core.cuh) of the residues, and no intermediate leaves the ranges
-// that the three-word form assumes (lazy::range_error).  Extreme words sit at every position.
+// that the three-word form assumes (lazy::range_error).  Extreme words sit at every position, and so
+// do the ends of the stated input range, +-2^65.
 #include <cstdint>
 #include <cstdio>
 #include <random>
@@ -18,16 +19,28 @@ static uint64_t pick(std::mt19937_64& rng) {
   return (r & 3) ? edge[(r >> 8) % 10] : rng();
 }
 
+// an end of the input range, or near it, and its residue
+static lazy::W3 bound(std::mt19937_64& rng, uint64_t& residue) {
+  __int128 v = lazy::kInputBound - (__int128)((rng() & 1) ? rng() % 3 : 0);
+  if (rng() & 1) v = -v;
+  const __int128 r = v % (__int128)gl::P;
+  residue = (uint64_t)(r < 0 ? r + gl::P : r);
+  return lazy::from_int(v);
+}
+
 template <int R>
 void check(std::mt19937_64& rng) {
-  for (int rep = 0; rep < 20000; ++rep) {
+  for (int rep = 0; rep < 25000; ++rep) {
     lazy::W3 x[R];
     uint64_t want[R], got[R];
-    const int mode = rep % 4;  // words of all extremes, products, one extreme value everywhere, +- halves
+    // words of all extremes, products, one extreme value everywhere, +- halves, ends of the input range
+    const int mode = rep % 5;
     const uint64_t all = pick(rng), other = pick(rng);
     for (int i = 0; i < R; ++i) {
       uint64_t a = mode == 2 ? all : (mode == 3 ? ((rng() & 1) ? all : other) : pick(rng));
-      if (mode == 1) {
+      if (mode == 4) {
+        x[i] = bound(rng, want[i]);
+      } else if (mode == 1) {
         const uint64_t b = pick(rng);
         x[i] = lazy::mul3(a, b);
         want[i] = gl::mul(canon(a), canon(b));
@@ -65,13 +78,14 @@ void check5(std::mt19937_64& rng) {
   const uint64_t w = gl::pow(554, (gl::P - 1) / 5);
   uint64_t c[4];
   lazy::dft5_constants(w, c);
-  for (int rep = 0; rep < 20000; ++rep) {
+  for (int rep = 0; rep < 30000; ++rep) {
     lazy::W3 u[5];
     uint64_t v[5], got[5];
     for (int i = 0; i < 5; ++i) {
       const uint64_t a = pick(rng), b = pick(rng);
-      u[i] = rep & 1 ? lazy::mul3(a, b) : lazy::from_word(a);
-      v[i] = rep & 1 ? gl::mul(canon(a), canon(b)) : canon(a);
+      const int mode = rep % 3;  // words, products, ends of the input range
+      u[i] = mode == 2 ? bound(rng, v[i]) : (mode ? lazy::mul3(a, b) : lazy::from_word(a));
+      if (mode != 2) v[i] = mode ? gl::mul(canon(a), canon(b)) : canon(a);
     }
     lazy::dft5(u, c, got);
     for (int k = 0; k < 5; ++k) {
