@@ -89,6 +89,7 @@ def lib() -> ctypes.CDLL:
         "lnt_shifted_words": ([u32, u32, ctypes.POINTER(u32), ctypes.POINTER(u32)], i32),
         "lnt_create": ([u32, u32, i32, i32, ctypes.POINTER(vp)], i32),
         "lnt_create_with_plan": ([u32, u32, i32, i32, ctypes.POINTER(PlanOptions), ctypes.POINTER(vp)], i32),
+        "lnt_runs_on_cluster": ([vp, ctypes.POINTER(i32)], i32),
         "lnt_get_plan": ([vp, ctypes.POINTER(PlanOptions)], i32),
         "lnt_plan_candidates": ([u32, u32, ctypes.POINTER(PlanOptions), i32, ctypes.POINTER(i32)], i32),
         "lnt_plan_describe": ([ctypes.POINTER(PlanOptions), u32, u32, cp, sz], i32),

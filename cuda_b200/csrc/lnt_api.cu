@@ -485,8 +485,13 @@ lnt::ClusterDesc cluster_desc(const lnt_test* t, uint64_t iterations) {
   return d;
 }
 
+// the cluster launch of this test alone (size 0: it runs on its plan's kernels)
+lnt::ClusterChoice lone_cluster(const lnt_test* t) {
+  return t->pw ? lnt::cluster_choice(t->n, t->n, 1) : lnt::ClusterChoice();
+}
+
 int queue_iterations(lnt_test* t, uint64_t iterations, LaunchTimer* timer) {
-  const lnt::ClusterChoice cl = t->pw ? lnt::cluster_choice(t->n, t->n, 1) : lnt::ClusterChoice();
+  const lnt::ClusterChoice cl = lone_cluster(t);
   if (cl.size) {
     const lnt::ClusterDesc d = cluster_desc(t, iterations);
     LNT_LAUNCH(lnt::launch_cluster(nullptr, d, 1, t->n, cl.size, cl.threads, cl.pass_log2, t->stream),
@@ -1452,6 +1457,13 @@ int lnt_get_plan(lnt_test* t, lnt_plan_options* out) {
   out->tile = p.kind == lnt::PlanKind::Resident ? 0 : p.tile;
   out->radix = p.fast ? p.radix : 0;
   out->fused = p.fast ? (p.fused ? 1 : 2) : 0;
+  return LNT_OK;
+}
+
+int lnt_runs_on_cluster(lnt_test* t, int* yes) {
+  if (!t || !yes) return fail(LNT_ERR_INVALID_ARGUMENT, "null argument");
+  DeviceGuard guard(t->device);
+  *yes = lone_cluster(t).size ? 1 : 0;
   return LNT_OK;
 }
 

@@ -242,6 +242,8 @@ void LucasPRP::DumpStats(double total_ms) {
     r.fft = std::to_string(n_);
     r.kernels = {"resident_square_loop"};
   }
+  int cluster = 0;
+  if (lnt_runs_on_cluster(t_, &cluster) == LNT_OK && cluster) r.kernels = {"cluster_square_loop"};
   r.performance_loops = o_.performance_loops;
   for (const Candidate& c : performances_)
     if (c.ms >= 0) r.performances.emplace_back(c.name, c.ms);

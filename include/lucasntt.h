@@ -94,7 +94,8 @@ int lnt_create(uint32_t exponent, uint32_t n, int prp, int device, lnt_test** ou
  * transpose tile, kernel.cu:157-192, :257-287). */
 typedef enum lnt_plan_kind {
   LNT_PLAN_AUTO = 0,     /* the policy's choice */
-  LNT_PLAN_RESIDENT = 1, /* n <= 4096: one CTA per residue, state in shared memory (FFT_1SMEM) */
+  LNT_PLAN_RESIDENT = 1, /* n <= 4096: the residue stays in shared memory for all squarings of a call
+                            (FFT_1SMEM): that of one CTA, or of a cluster (below) */
   LNT_PLAN_RADIX16 = 2,  /* 4-step columns x rows, register passes of radix <= 16 (FFT_2SMEM family) */
   LNT_PLAN_RADIX2 = 3    /* 4-step columns x rows, radix-2 stages (the first kernels; an explicit plan) */
 } lnt_plan_kind;
@@ -104,7 +105,9 @@ typedef struct lnt_plan_options {
   uint32_t log2_rows; /* two-pass: log2 of the column length n2 (n = n2 x n1); 0 = policy */
   uint32_t tile;      /* two-pass: columns per column CTA = words per carry run, 4 or 8; 0 = policy */
   uint32_t radix;     /* LNT_PLAN_RADIX16: largest pass radix, 8 or 16; 0 = policy
-                         (16 from 2^19 words) */
+                         (16 from 2^19 words).  16: columns of 1024 words and more take passes
+                         of 16 points, and rows of 1024 and 2048 words do in launches that
+                         leave registers idle; the other passes take 8 points */
   uint32_t fused;     /* LNT_PLAN_RADIX16: 1 = the inverse column pass of a squaring and the
                          forward one of the next in one carry-fused launch, 2 = two launches;
                          0 = policy (fused from 2^19 words) */
@@ -119,6 +122,12 @@ int lnt_create_with_plan(uint32_t exponent, uint32_t n, int prp, int device,
 
 /* The plan a test runs. */
 int lnt_get_plan(lnt_test* t, lnt_plan_options* out);
+
+/* *yes = 1 if the squarings of this test alone run on the cluster kernel
+ * (cluster_square_loop): 512 to 32768 words spread over the shared memories of
+ * a cluster's CTAs.  It serves the policy's plan of such a length, however that
+ * plan was chosen, under that plan's name; batches use it for few small tests. */
+int lnt_runs_on_cluster(lnt_test* t, int* yes);
 
 /* KernelFactory::GetCandidates analogue (kernel_factory.cu:45-141): every valid
  * plan for (q, n) (n = 0: policy length).  Writes min(count, cap) entries. */

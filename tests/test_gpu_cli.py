@@ -226,3 +226,14 @@ def test_five_length_from_the_ini(tmp_path):
     assert "not optimal" in r.stdout and "M(216091) is prime!" in r.stdout
     s = stats(tmp_path / "LucasNTT_results.txt")
     assert s["Res64"] == "0000000000000000" and s["fft"] == "64:640"
+
+
+@pytest.mark.parametrize("q,n,kernel", [(1279, 64, "resident_square_loop"), (44497, 2048, "cluster_square_loop"),
+                                        (160001, 8192, "cluster_square_loop")])
+def test_stats_name_the_kernel_that_ran(lnt, tmp_path, q, n, kernel):
+    r = run_cli(tmp_path, [q, 100], ini=f"fft = {n}\nPerformanceLoops = 50\n", stdin="y\n")
+    assert r.returncode == 0, r.stdout + r.stderr
+    with lnt.LucasTest(q, n) as t:
+        assert list(t.profile_iterations(1)) == [kernel]
+    text = (tmp_path / "LucasNTT_results.txt").read_text()
+    assert f"Kernel0 = {kernel}" in text and "Kernel1" not in text
