@@ -34,7 +34,6 @@
 #include <stdint.h>
 
 #include "goldilocks.cuh"
-#include "ntt_core.cuh"
 
 namespace lnt {
 namespace lazy {

@@ -12,7 +12,7 @@
 // (the last one writes to the natural owners), inverse radix-C pass, unweight and carry runs: three
 // exchanges and about eight CTA barriers, no global memory access.  (With cluster barriers in place
 // of the counted stores of `send`: 5.45 us against 5.09 at n = 2048.)  Twiddles, weights and
-// unweights sit in shared memory (66 bytes a word: up to m = 2048).
+// unweights sit in shared memory (69 bytes a word with the two buffers: up to m = 2048).
 //
 // Replaces the reference's FFT_1SMEM pool as lnt_resident.cu does (kernel_pool.cu:31-38).
 #include <algorithm>
@@ -180,7 +180,7 @@ template <int C>
 __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __restrict__ descs,
                                                              const __grid_constant__ ClusterDesc one, int pass_log2) {
   extern __shared__ __align__(16) uint64_t sm[];
-  constexpr int kLogC = C == 2 ? 1 : (C == 4 ? 2 : (C == 8 ? 3 : 4));
+  constexpr int kLogC = C == 4 ? 2 : (C == 8 ? 3 : 4);
   const ClusterDesc& D = descs ? descs[blockIdx.x / C] : one;
   const uint32_t rank = cluster_rank();
   const int n = (int)D.n, m = n / C, seg = m / C, lseg = __ffs(seg) - 1;
@@ -452,14 +452,14 @@ int max_clusters() {
 
 }  // namespace
 
+namespace {
 bool cluster_fits(uint32_t n, uint32_t C) {
   // segments hold whole 8-word runs, blocks at least two passes and at most 2048 words
   return n >= 8 * C * C && n / C >= 64 && n / C <= 2048;
 }
 
-int cluster_max_active(uint32_t C) {
-  return C == 4 ? max_clusters<4>() : (C == 8 ? max_clusters<8>() : (C == 16 ? max_clusters<16>() : 0));
-}
+int cluster_max_active(uint32_t C) { return C == 4 ? max_clusters<4>() : (C == 8 ? max_clusters<8>() : max_clusters<16>()); }
+}  // namespace
 
 // One B200, us a squaring of one test alone, against the resident (to 4096) or two-pass kernels:
 //   n        512    1024    2048    4096    8192   16384   32768

@@ -143,7 +143,6 @@ struct ClusterChoice {
   int threads = 0, pass_log2 = 3;
 };
 ClusterChoice cluster_choice(uint32_t min_n, uint32_t max_n, uint32_t count);
-bool cluster_fits(uint32_t n, uint32_t C);
 // descs == nullptr: the one test `one`
 cudaError_t launch_cluster(const ClusterDesc* descs, const ClusterDesc& one, uint32_t count, uint32_t max_n,
                            uint32_t C, int threads, int pass_log2, cudaStream_t s);

@@ -16,7 +16,6 @@
 
 #include "carry.cuh"
 #include "lnt_internal.h"
-#include "ntt_core.cuh"
 #include "smem_passes.cuh"
 
 namespace lnt {
@@ -255,7 +254,7 @@ __global__ void __launch_bounds__(TH) row_mul_r16(const TwoPassDesc* __restrict_
 // Mode 0: square (a squaring), 1: forward only (the operand F of a product,
 // left in x in plane-major order), 2: product with F.  A CTA takes `rows`
 // consecutive rows: plane k5 of row g at sm + (5 g + k5) ld.
-template <int TH, int MR, int Mode>
+template <int TH, int Mode>
 __global__ void __launch_bounds__(TH) row5_r16(const TwoPassDesc* __restrict__ Ds, Passes P, int rows,
                                                const uint64_t* __restrict__ F) {
   extern __shared__ __align__(16) uint64_t sm[];
@@ -285,7 +284,7 @@ __global__ void __launch_bounds__(TH) row5_r16(const TwoPassDesc* __restrict__ D
   int span = L;
   const int last = Mode == 1 ? P.m : P.m - 1;
   for (int j = 0, seg = 0; j < last; ++j) {
-    pass_r<0, MR>(P.radix[j], sm, ld, 5 * rows, L, span, D.itw1 + seg);
+    pass_r<0>(P.radix[j], sm, ld, 5 * rows, L, span, D.itw1 + seg);
     seg += span;
     span /= P.radix[j];
     __syncthreads();
@@ -298,13 +297,13 @@ __global__ void __launch_bounds__(TH) row5_r16(const TwoPassDesc* __restrict__ D
   } else {
     // last forward pass, square (or product with F) and first inverse pass
     if constexpr (Mode == 0)
-      pass_r<2, MR>(P.radix[P.m - 1], sm, ld, 5 * rows, L, span, nullptr);
+      pass_r<2>(P.radix[P.m - 1], sm, ld, 5 * rows, L, span, nullptr);
     else
-      pass_r<3, MR>(P.radix[P.m - 1], sm, ld, 5 * rows, L, span, F + off);
+      pass_r<3>(P.radix[P.m - 1], sm, ld, 5 * rows, L, span, F + off);
     __syncthreads();
     for (int j = P.m - 2; j >= 0; --j) {
       span *= P.radix[j];
-      pass_r<1, MR>(P.radix[j], sm, ld, 5 * rows, L, span, D.iitw1 + pass_table_offset(P, L, j));
+      pass_r<1>(P.radix[j], sm, ld, 5 * rows, L, span, D.iitw1 + pass_table_offset(P, L, j));
       __syncthreads();
     }
     // planes -> HBM: inverse twiddle, inverse 5-point transform, inverse 4-step twiddle
@@ -854,10 +853,10 @@ cudaError_t row5_launch(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t co
     kernel<<<grid, th, smem, s>>>(dd, P, rows, F);
     return cudaGetLastError();
   };
-  if (words <= 1280) return go(row5_r16<128, 8, Mode>, 128);
-  if (words <= 5120) return go(row5_r16<256, 8, Mode>, 256);
-  if (words <= 10240) return go(row5_r16<512, 8, Mode>, 512);
-  return go(row5_r16<1024, 8, Mode>, 1024);
+  if (words <= 1280) return go(row5_r16<128, Mode>, 128);
+  if (words <= 5120) return go(row5_r16<256, Mode>, 256);
+  if (words <= 10240) return go(row5_r16<512, Mode>, 512);
+  return go(row5_r16<1024, Mode>, 1024);
 }
 
 cudaError_t launch_row_forward_r16(const TwoPassDesc& d, const TwoPassDesc* dd, cudaStream_t s) {

@@ -1,13 +1,13 @@
-// Register-resident NTTs of up to 64 points with power-of-two roots.
+// Register-resident NTTs of up to 64 points with power-of-two roots, canonical after every step.
+// The kernels run the lazily reduced transforms of lazy_core.cuh; these are what the self-tests
+// compare those with.
 //
 // In F_p, 2 has order 192 and 554^((p-1)/64) = 2^3, so the R-point root used by
 // every sub-transform of the reference's roots (pre_calculation.cu:61-66) with
 // R | 64 is omega_R = 2^(192/R): each butterfly twiddle is a multiplication by
 // a power of two, done with shifts and adds (shl_c), never the multiplier.  The
 // reference reaches this only for its radix-4/8 inner roots and its 32x32 row
-// kernel (kernels/fftr_sqr_ifftr__r2_32x32_1024.cu); here every transform of
-// length L = 64 * R is split into register passes of 64 and R points with one
-// table-twiddle level between them.
+// kernel (kernels/fftr_sqr_ifftr__r2_32x32_1024.cu).
 //
 // dif<R>: natural order in, bit-reversed order out (decimation in frequency).
 // dit_inv<R>: bit-reversed in, natural out, inverse roots, unscaled.

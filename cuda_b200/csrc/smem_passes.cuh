@@ -5,7 +5,7 @@
 // A transform of length L = r0 * r1 * ... (every r a power of two) runs as
 // passes over shared memory: pass j takes R = r_j elements at stride span_j / R
 // from a block of span_j = L / (r0 ... r_{j-1}) words into registers, does an
-// R-point DIF with power-of-two twiddles (ntt_core.cuh), multiplies by
+// R-point DIF with power-of-two twiddles (lazy_core.cuh), multiplies by
 // omega_span^(t * k) and writes back.  The result is in fully bit-reversed
 // order; the inverse passes (DIT) take it back to natural order.  Per element a
 // pass costs log2(R) shift butterflies and one table multiplication; the
@@ -15,7 +15,8 @@
 // Small unrolled bodies (one R-point transform) inside runtime loops keep the
 // kernels small enough for the instruction cache; fully unrolled 64-point
 // passes starved the SM of instructions.  Shared memory is padded by one word
-// in 16 (sw below), which makes every pass stride bank-conflict free.
+// in 16 (sw below), which makes the pass strides bank-conflict free, q = 8 of an
+// 8-point pass excepted (swap_tasks).
 #pragma once
 #include <stdint.h>
 

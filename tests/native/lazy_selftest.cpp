@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <random>
 #include "../../cuda_b200/csrc/lazy_core.cuh"
+#include "../../cuda_b200/csrc/ntt_core.cuh"
 
 using namespace lnt;
 static int fails = 0;
