@@ -399,17 +399,6 @@ __device__ __forceinline__ void load_colf(const TwoPassDesc& D, uint32_t t0, uin
   }
 }
 
-// Short columns (a row or two per thread; one test alone): touch this tile's factors while its words
-// are on their way, so that the carry steps find them in the L1.
-__device__ __forceinline__ void warm_factors(const TwoPassDesc& D, uint32_t c0) {
-  const int L = (int)D.n2;
-  if (L > 512) return;
-  uint32_t u;
-  for (int r = threadIdx.x; r < L; r += blockDim.x)
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(u) : "l"(D.rowf + 2 * r));
-  if (threadIdx.x == 0) asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(u) : "l"(D.colf + c0));
-}
-
 // A row of a tile, as 16-byte vectors.
 template <int T>
 __device__ __forceinline__ void load_row(const uint64_t* row, uint64_t (&v)[T]) {
@@ -539,7 +528,6 @@ __global__ void __launch_bounds__(TH, min_blocks<TH, MR>()) col_forward_r16(
   extern __shared__ __align__(16) uint64_t sm[];
   const TwoPassDesc& D = Ds[blockIdx.y];
   uint32_t status = 0;
-  warm_factors(D, blockIdx.x * T);
   tile_load<T>(sm, D.x, (int)D.n2, D.n1, blockIdx.x * T);
   __syncthreads();
   forward_tile<T, MR>(D, P, sm, blockIdx.x, apply_carries != 0, false, status);
@@ -551,7 +539,6 @@ __global__ void __launch_bounds__(TH, min_blocks<TH, MR>()) col_inverse_r16(
     const TwoPassDesc* __restrict__ Ds, Passes P, int unsigned_mode) {
   extern __shared__ __align__(16) uint64_t sm[];
   const TwoPassDesc& D = Ds[blockIdx.y];
-  warm_factors(D, blockIdx.x * T);
   tile_load<T>(sm, D.x, (int)D.n2, D.n1, blockIdx.x * T);
   __syncthreads();
   inverse_tile<T, MR>(D, P, sm, blockIdx.x, unsigned_mode != 0);
@@ -650,7 +637,6 @@ __global__ void __launch_bounds__(TH, min_blocks<TH, MR, Dense>()) col_fused_r16
   for (int i = 0; i < ninv; ++i) {
     const bool lasttile = ticket == 0 && i == 0;
     const uint32_t tile = lasttile ? last : ticket;
-    warm_factors(D, tile * T);
     tile_load<T>(sm, D.x, L, n1, tile * T);
     __syncthreads();
     inverse_tile<T, MR>(D, P, sm, tile, false);
@@ -925,8 +911,10 @@ cudaError_t col_fused_t(const TwoPassDesc& d, const TwoPassDesc* dd, uint32_t co
 
 // 16-point passes of 4-word tiles up to 2048 rows (73 KB: three fit an SM): three CTAs an SM instead
 // of two where the launch has eight tiles an SM and more.  col_fused, two -> three, us: 2560 tiles of 1024
-// rows (n = 5 * 2^21) 246.7 -> 223.2, 1024 of 2048 (2^23) 180.4 -> 177.9; 512 of 2048 (2^22) 108.0 -> 113.3,
-// 512 of 1024 (2^21) 59.2 -> 65.8, where the third CTA saves no wave.
+// rows (n = 5 * 2^21) 246.7 -> 223.2; 512 of 2048 (2^22) 108.0 -> 113.3, 512 of 1024 (2^21) 59.2 -> 65.8, where
+// the third CTA saves no wave.  The line keeps clear of those: 1024 tiles of 2048 (one test at 2^23) lie below it
+// and take two, although three would be 180.9 -> 177.6 there; other launches of 600 to 1184 tiles
+// (several tests) have not been measured.
 bool col_dense(const TwoPassDesc& d, uint32_t count) {
   return d.tile == 4 && d.n2 <= 2048 && (uint64_t)d.ntiles * count >= 8ull * device_sms();
 }
