@@ -58,9 +58,10 @@ def test_pending_carries_of_the_two_pass_kernels(lnt):
         assert a.gerbicz_stats()["checks"] >= 3 and a.gerbicz_stats()["errors"] == 0
 
 
-@pytest.mark.parametrize("count", [1, 7, 24, 60])
+@pytest.mark.parametrize("count", [1, 7, 24, 60, 160])
 def test_batches_of_every_cluster_size(lnt, count):
-    """Mixed lengths in one launch: clusters of eight, four, and one CTA per test."""
+    """Mixed lengths in one launch: clusters of eight, four, and one CTA per test (fewer tests than SMs, and
+    more), against the same tests alone."""
     qs = [(9689, 21701, 44021, 86243)[i % 4] + 2 * i for i in range(count)]
     with lnt.Batch() as b:
         ids = [b.submit(q, prp=bool(i & 1), iterations=300) for i, q in enumerate(qs)]
