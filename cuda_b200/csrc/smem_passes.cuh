@@ -15,8 +15,7 @@
 // Small unrolled bodies (one R-point transform) inside runtime loops keep the
 // kernels small enough for the instruction cache; fully unrolled 64-point
 // passes starved the SM of instructions.  Shared memory is padded by one word
-// in 16 (sw below), which makes the pass strides bank-conflict free, q = 8 of an
-// 8-point pass excepted (swap_tasks).
+// in 16 (sw below), or laid out as Tile.
 #pragma once
 #include <stdint.h>
 
@@ -33,7 +32,9 @@ __host__ __device__ constexpr int padded(int L) { return L + L / 16; }
 // one word of padding in 16.  Tile<T>: T transforms interleaved, word (i, g) at T (i + i / 8) + g, so a
 // row of T words stays together: it is copied 16 bytes at a time, read as vectors by the carry
 // steps, and T neighbouring threads share their twiddles.  Both layouts keep off + q d at a
-// constant stride in d (q >= 16, or 8 for Tile) and every pass free of bank conflicts.
+// constant stride in d (q >= 16, or 8 for Tile) and, with the task order of swap_tasks, keep passes of up
+// to 8 points free of bank conflicts; a 16-point pass of stride 1 in a tile of four columns reads
+// words 72 apart, which collide two ways.
 struct Rows {
   static constexpr int kStride = 1, kPadLog2 = 4, kTile = 1;
 };
