@@ -271,7 +271,8 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
   // exchanges that this CTA sent, and that it received and re-armed, when it leaves the loop
   uint64_t sent = 0, passed = 0;
   bool lost = false;  // this CTA gave up
-  for (uint64_t it = 0; it < D.iterations; ++it) {
+  const uint64_t stop = rank == 0 && D.quit_at < D.iterations ? D.quit_at : D.iterations;
+  for (uint64_t it = 0; it < stop; ++it) {
     const bool um = D.unsigned_first && it == 0;
     // carry-in of the run before, then weight
     for (int i = tid; i < runs; i += bd) {
@@ -283,10 +284,9 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
         v = lazy::mul_digit((int64_t)v, S.w[sw(i * K + k)]);
       }
     }
-    if (rank == 0 && it == D.quit_at) status |= kStatusClusterTimeout;
-    if ((lost = gave_up(status))) {
+    if ((lost = gave_up(status))) {  // of the exchange before: no wait has run when it = 0
       sent = 3 * it;
-      passed = it ? sent - 1 : 0;
+      passed = sent - 1;
       break;
     }
     if (it && tid == 0) expect_bytes(S.bar + 2, 8u * (uint32_t)C);
@@ -366,9 +366,10 @@ __global__ void __launch_bounds__(512) cluster_square_loop(const ClusterDesc* __
     await_phase(S.bar + 2, parity, D.wait_ns, status);
   }
   if (!lost) {
+    if (stop < D.iterations) status |= kStatusClusterTimeout;
     lost = gave_up(status);
-    sent = 3 * D.iterations;
-    passed = lost ? sent - 1 : sent;
+    sent = 3 * stop;
+    passed = lost && sent ? sent - 1 : sent;
   }
 
   if (!lost) {
@@ -467,6 +468,7 @@ int cluster_max_active(uint32_t C) { return C == 4 ? max_clusters<4>() : (C == 8
 //   C = 4   4.42    4.57    5.46    6.81    10.0     -       -
 //   C = 8   4.54    5.00    5.09    5.88    7.14    10.2     -
 //   C = 16   -       -      7.20    7.29    8.01    9.17    11.8
+//   now     4.05    4.13    4.68    5.54    6.86    8.53    11.1   (the size taken; the rows above are older)
 // About 4 us are the latency of a dozen phases of one or two warps per scheduler.  Local passes of
 // radix 4 beat radix 8 (half as long for two of the three stages) up to blocks of 1024 words.
 // A launch of several tests takes the largest size of which the GPU holds all clusters at once; where
